@@ -90,6 +90,12 @@ struct DeviceSceneBuffers {
     void*    env_pmf = nullptr;
     void*    env_alias = nullptr;
     void*    punctual = nullptr;
+    void*    wide = nullptr;               // four-wide tree (wide.h): nodes, triangle records
+    void*    wtris = nullptr;
+    size_t   wide_bytes = 0, wtris_bytes = 0;
+    bool     wide_on = false;
+    uint32_t wide_root = 0, wide_need = 0; // root reference; stack entries its walk may need
+    float    coord_max[3] = {0, 0, 0};
     void*    env_array = nullptr;          // cudaArray_t
     unsigned long long env_tex = 0;        // cudaTextureObject_t
     std::vector<void*> tex_arrays;         // per material texture: cudaArray_t (null when empty)

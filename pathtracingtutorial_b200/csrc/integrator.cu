@@ -20,6 +20,8 @@
 // sequence that is captured once into a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -30,6 +32,7 @@
 #include "engine.h"
 #include "bsdf.h"
 #include "traverse.h"
+#include "wide.h"
 #include <cub/device/device_scan.cuh>
 
 #include "guide.cuh"
@@ -389,11 +392,22 @@ __device__ __forceinline__ void warp_count(unsigned long long* dst, uint32_t v) 
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(dst, static_cast<unsigned long long>(v));
 }
 
-// Closest hits of queue q.  Packet: the queue holds camera rays, 32
-// neighbouring pixels of one sample per warp, walked as packets
-// (closest_packet_loop); else lane by lane with refill (closest_loop).
-template <int Block, int Depth, bool Packet = false>
-__global__ void __launch_bounds__(Block) k_extend(WaveParams P, int q, int depth) {
+// How a traversal kernel walks its rays.
+enum TraceMode {
+    kTraceBinary = 0,       // binary tree: traversal counters, scenes without a wide tree
+    kTraceWide,             // four-wide tree
+    kTraceWideWatertight,
+    kTraceModes
+};
+
+// Closest hits of queue q.
+// Resident blocks the wide kernels are compiled for: 8 of 128 threads (64
+// registers; left to itself the compiler takes 72 and the closed room's
+// extension stage 101 instead of 97 ms; 56 registers: 97 ms).
+constexpr int wide_blocks(int block, int mode) { return mode == kTraceBinary ? 0 : 1024 / block; }
+
+template <int Block, int Depth, int Mode>
+__global__ void __launch_bounds__(Block, wide_blocks(Block, Mode)) k_extend(WaveParams P, int q, int depth) {
     const uint32_t n = min(P.counts[q], static_cast<uint32_t>(P.npath));
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         P.counts[q ^ 1] = 0;
@@ -401,11 +415,7 @@ __global__ void __launch_bounds__(Block) k_extend(WaveParams P, int q, int depth
         P.counts[4] = 0;
         atomicAdd(P.stats + (depth == 0 ? kStatCameraRays : kStatExtRays), static_cast<unsigned long long>(n));
     }
-    const bool watertight = (P.flags & PT_FLAG_WATERTIGHT) != 0;
-    const bool count = (P.flags & PT_FLAG_COUNT_TRAVERSAL) != 0;
     uint32_t err = 0;
-    TraceCounters tc{0, 0};
-    const uint32_t stride = gridDim.x * blockDim.x;
     const float4* __restrict__ ro = P.ray_o[q];
     const float4* __restrict__ rd = P.ray_d[q];
     float4* __restrict__ hit = P.hit;
@@ -414,21 +424,27 @@ __global__ void __launch_bounds__(Block) k_extend(WaveParams P, int q, int depth
         const float4 d = rd[i];
         r = make_ray_inv(o.x, o.y, o.z, d.x, d.y, d.z);
     };
-    auto done = [&](uint32_t i, const ClosestWalk& w) {
-        hit[i] = w.prim >= 0 ? make_float4(w.best, __int_as_float(w.prim), w.bu, w.bv)
-                             : make_float4(FLT_MAX, __int_as_float(-1), 0.0f, 0.0f);
-    };
-    if (Packet) {
-        closest_packet_loop<Depth>(P.scene, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, stride >> 5, n, watertight,
-                                   err, tc, fetch, done);
+    if constexpr (Mode == kTraceWide || Mode == kTraceWideWatertight) {
+        wide_closest_loop<Depth, Mode == kTraceWideWatertight>(
+            P.scene, n, err, fetch, [&](uint32_t i, int prim, float t, float u, float v) {
+                hit[i] = prim >= 0 ? make_float4(t, __int_as_float(prim), u, v)
+                                   : make_float4(FLT_MAX, __int_as_float(-1), 0.0f, 0.0f);
+            });
+        if (err) atomicOr(P.err, err);
     } else {
-        closest_loop<Depth>(P.scene, blockIdx.x * blockDim.x + threadIdx.x, n, stride, watertight, err, tc, fetch,
-                            done);
-    }
-    if (err) atomicOr(P.err, err);
-    if (count) {
-        warp_count(P.stats + kStatNodes, tc.inner);
-        warp_count(P.stats + kStatTris, tc.tris);
+        const bool watertight = (P.flags & PT_FLAG_WATERTIGHT) != 0;
+        TraceCounters tc{0, 0};
+        auto done = [&](uint32_t i, const ClosestWalk& w) {
+            hit[i] = w.prim >= 0 ? make_float4(w.best, __int_as_float(w.prim), w.bu, w.bv)
+                                 : make_float4(FLT_MAX, __int_as_float(-1), 0.0f, 0.0f);
+        };
+        closest_loop<Depth>(P.scene, blockIdx.x * blockDim.x + threadIdx.x, n, gridDim.x * blockDim.x, watertight, err,
+                            tc, fetch, done);
+        if (err) atomicOr(P.err, err);
+        if (P.flags & PT_FLAG_COUNT_TRAVERSAL) {
+            warp_count(P.stats + kStatNodes, tc.inner);
+            warp_count(P.stats + kStatTris, tc.tris);
+        }
     }
 }
 
@@ -907,25 +923,13 @@ __global__ void __launch_bounds__(128, 6) k_shade_back(WaveParams P, int q, int 
     }
 }
 
-// Any-hit tests of the shadow queue.  Packet: the queue holds the shadow rays
-// of the camera bounce, emitted warp by warp from neighbouring pixels, tested
-// as packets where a tile's directions share their signs (any_packet_loop).
-template <int Block, int Depth, bool Packet = false>
-__global__ void __launch_bounds__(Block) k_shadow(WaveParams P) {
+// Any-hit tests of the shadow queue.
+template <int Block, int Depth, int Mode>
+__global__ void __launch_bounds__(Block, wide_blocks(Block, Mode)) k_shadow(WaveParams P) {
     const uint32_t n = min(P.counts[2], static_cast<uint32_t>(P.npath) * static_cast<uint32_t>(P.n_slots));
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(P.stats + kStatShadowRays, static_cast<unsigned long long>(n));
-    const bool watertight = (P.flags & PT_FLAG_WATERTIGHT) != 0;
-    const bool count = (P.flags & PT_FLAG_COUNT_TRAVERSAL) != 0;
     uint32_t err = 0;
-    TraceCounters tc{0, 0};
-    const uint32_t stride = gridDim.x * blockDim.x;
-    auto fetch = [&](uint32_t i, AnyWalk& w) {
-        const float4 o = P.sq_o[i];
-        const float4 d = P.sq_d[i];
-        w.r = make_ray_inv(o.x, o.y, o.z, d.x, d.y, d.z);
-        w.tmax = d.w;
-    };
     auto done = [&](uint32_t i, bool occluded) {
         if (occluded) return;
         const uint32_t slot = __float_as_uint(P.sq_o[i].w);
@@ -940,15 +944,33 @@ __global__ void __launch_bounds__(Block) k_shadow(WaveParams P) {
             err |= kErrQueueOverflow;
         }
     };
-    if (Packet)
-        any_packet_loop<Depth>(P.scene, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, stride >> 5, n, watertight, err,
-                               tc, fetch, done);
-    else
-        any_loop<Depth>(P.scene, blockIdx.x * blockDim.x + threadIdx.x, n, stride, watertight, err, tc, fetch, done);
-    if (err) atomicOr(P.err, err);
-    if (count) {
-        warp_count(P.stats + kStatShadowNodes, tc.inner);
-        warp_count(P.stats + kStatShadowTris, tc.tris);
+    if constexpr (Mode == kTraceWide || Mode == kTraceWideWatertight) {
+        wide_any_loop<Depth, Mode == kTraceWideWatertight>(
+            P.scene, n, err,
+            [&](uint32_t i, RayInv& r) {
+                const float4 o = P.sq_o[i];
+                const float4 d = P.sq_d[i];
+                r = make_ray_inv(o.x, o.y, o.z, d.x, d.y, d.z);
+                return d.w;
+            },
+            done);
+        if (err) atomicOr(P.err, err);
+    } else {
+        const bool watertight = (P.flags & PT_FLAG_WATERTIGHT) != 0;
+        TraceCounters tc{0, 0};
+        auto fetch = [&](uint32_t i, AnyWalk& w) {
+            const float4 o = P.sq_o[i];
+            const float4 d = P.sq_d[i];
+            w.r = make_ray_inv(o.x, o.y, o.z, d.x, d.y, d.z);
+            w.tmax = d.w;
+        };
+        any_loop<Depth>(P.scene, blockIdx.x * blockDim.x + threadIdx.x, n, gridDim.x * blockDim.x, watertight, err, tc,
+                        fetch, done);
+        if (err) atomicOr(P.err, err);
+        if (P.flags & PT_FLAG_COUNT_TRAVERSAL) {
+            warp_count(P.stats + kStatShadowNodes, tc.inner);
+            warp_count(P.stats + kStatShadowTris, tc.tris);
+        }
     }
 }
 
@@ -1064,35 +1086,40 @@ __global__ void k_film_mean(const float4* sum, const float4* comp, float4* out, 
 }
 
 // ---- diagnostics ----
-__global__ void k_trace_rays(DeviceScene s, const float* rays, uint32_t n, pt_hit* hits, uint8_t* occl,
-                             int any, int watertight, uint32_t* err_out) {
-    // the warp-scheduled loops of the wavefront kernels
+// Closest hits (Any = false) or occlusion of a ray buffer, by the walks of the
+// wavefront kernels.
+template <int Depth, int Mode, bool Any>
+__global__ void __launch_bounds__(128, wide_blocks(128, Mode)) k_trace_rays(DeviceScene s, const float* rays, uint32_t n, pt_hit* hits,
+                                                    uint8_t* occl, int watertight, uint32_t* err_out) {
     uint32_t err = 0;
     TraceCounters tc{0, 0};
     const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     const float4* r4 = reinterpret_cast<const float4*>(rays);
-    if (any) {
-        any_loop(s, first, n, stride, watertight != 0, err, tc,
-                 [&](uint32_t i, AnyWalk& w) {
-                     const float4 o = r4[2 * i], d = r4[2 * i + 1];
-                     w.r = make_ray_inv(o.x, o.y, o.z, d.x, d.y, d.z);
-                     w.tmax = d.w;
-                 },
-                 [&](uint32_t i, bool occluded) { occl[i] = occluded ? 1 : 0; });
+    auto ray = [&](uint32_t i, RayInv& r) {
+        const float4 o = r4[2 * static_cast<size_t>(i)], d = r4[2 * static_cast<size_t>(i) + 1];
+        r = make_ray_inv(o.x, o.y, o.z, d.x, d.y, d.z);
+        return d.w;
+    };
+    auto occluded = [&](uint32_t i, bool hit) { occl[i] = hit ? 1 : 0; };
+    auto store = [&](uint32_t i, int prim, float t, float u, float v) {
+        pt_hit h;
+        h.prim = prim;
+        h.t = prim >= 0 ? t : FLT_MAX;
+        h.u = prim >= 0 ? u : 0.0f;
+        h.v = prim >= 0 ? v : 0.0f;
+        hits[i] = h;
+    };
+    if (Mode == kTraceBinary) {
+        if (Any)
+            any_loop(s, first, n, stride, watertight != 0, err, tc,
+                     [&](uint32_t i, AnyWalk& w) { w.tmax = ray(i, w.r); }, occluded);
+        else
+            closest_loop(s, first, n, stride, watertight != 0, err, tc, ray,
+                         [&](uint32_t i, const ClosestWalk& w) { store(i, w.prim, w.best, w.bu, w.bv); });
+    } else if (Any) {
+        wide_any_loop<Depth, Mode == kTraceWideWatertight>(s, n, err, ray, occluded);
     } else {
-        closest_loop(s, first, n, stride, watertight != 0, err, tc,
-                     [&](uint32_t i, RayInv& r) {
-                         const float4 o = r4[2 * i], d = r4[2 * i + 1];
-                         r = make_ray_inv(o.x, o.y, o.z, d.x, d.y, d.z);
-                     },
-                     [&](uint32_t i, const ClosestWalk& w) {
-                         pt_hit h;
-                         h.prim = w.prim;
-                         h.t = w.prim >= 0 ? w.best : FLT_MAX;
-                         h.u = w.prim >= 0 ? w.bu : 0.0f;
-                         h.v = w.prim >= 0 ? w.bv : 0.0f;
-                         hits[i] = h;
-                     });
+        wide_closest_loop<Depth, Mode == kTraceWideWatertight>(s, n, err, ray, store);
     }
     if (err) atomicOr(err_out, err);
 }
@@ -1121,54 +1148,55 @@ __global__ void k_bsdf_eval(const pt_material* mats, uint32_t nmat, const float*
     }
 }
 
-// The traversal kernels' shapes: 64, 128 or 256 threads per block and a
-// stack of 32 or 64 entries (six instantiations of k_extend and k_shadow).
+// The traversal kernels' shapes: 64, 128 or 256 threads per block with a stack
+// of 32 or 64 entries, and 128 threads with kDeepStack entries for four-wide
+// trees that need more.
+constexpr int kDeepStack = 192;   // three deferred children a level of the deepest tree accepted
+constexpr int kTraceShapes = 7;
 inline int trace_shape_index(int block, int depth) {
+    if (depth > 64) return 6;
     return (block == 64 ? 0 : (block == 256 ? 2 : 1)) * 2 + (depth == 32 ? 0 : 1);
 }
-inline int trace_shape_block(int k) { return k < 2 ? 64 : (k < 4 ? 128 : 256); }
-inline int trace_shape_depth(int k) { return (k & 1) ? 64 : 32; }
+inline int trace_shape_block(int k) { return k == 6 ? 128 : (k < 2 ? 64 : (k < 4 ? 128 : 256)); }
 
-#define PT_TRACE_SHAPES(X) X(0, 64, 32) X(1, 64, 64) X(2, 128, 32) X(3, 128, 64) X(4, 256, 32) X(5, 256, 64)
+using ExtendKernel = void (*)(WaveParams, int, int);
+using ShadowKernel = void (*)(WaveParams);
 
-inline const void* extend_kernel(int k) {
+// Kernel of a mode and shape.  The binary walk comes in one shape, the
+// watertight one in the two stack sizes.
+template <int Mode>
+ExtendKernel extend_shape(int k) {
     switch (k) {
-#define PT_CASE(i, b, d) case i: return reinterpret_cast<const void*>(k_extend<b, d>);
-        PT_TRACE_SHAPES(PT_CASE)
-#undef PT_CASE
-    }
-    return reinterpret_cast<const void*>(k_extend<128, 64>);
-}
-inline const void* shadow_kernel(int k) {
-    switch (k) {
-#define PT_CASE(i, b, d) case i: return reinterpret_cast<const void*>(k_shadow<b, d>);
-        PT_TRACE_SHAPES(PT_CASE)
-#undef PT_CASE
-    }
-    return reinterpret_cast<const void*>(k_shadow<128, 64>);
-}
-inline void launch_extend(int k, int grid, cudaStream_t st, const WaveParams& P, int q, int d) {
-    switch (k) {
-#define PT_CASE(i, b, dd)                                                   \
-    case i:                                                                 \
-        if (d == 0) k_extend<b, dd, true><<<grid, b, 0, st>>>(P, q, d);     \
-        else k_extend<b, dd><<<grid, b, 0, st>>>(P, q, d);                  \
-        return;
-        PT_TRACE_SHAPES(PT_CASE)
-#undef PT_CASE
+        case 0: return k_extend<64, 32, Mode>;
+        case 1: return k_extend<64, 64, Mode>;
+        case 2: return k_extend<128, 32, Mode>;
+        case 4: return k_extend<256, 32, Mode>;
+        case 5: return k_extend<256, 64, Mode>;
+        default: return k_extend<128, 64, Mode>;
     }
 }
-inline void launch_shadow(int k, int grid, cudaStream_t st, const WaveParams& P, int depth) {
+template <int Mode>
+ShadowKernel shadow_shape(int k) {
     switch (k) {
-#define PT_CASE(i, b, d)                                                    \
-    case i:                                                                 \
-        if (depth == 0) k_shadow<b, d, true><<<grid, b, 0, st>>>(P);        \
-        else k_shadow<b, d><<<grid, b, 0, st>>>(P);                         \
-        return;
-        PT_TRACE_SHAPES(PT_CASE)
-#undef PT_CASE
+        case 0: return k_shadow<64, 32, Mode>;
+        case 1: return k_shadow<64, 64, Mode>;
+        case 2: return k_shadow<128, 32, Mode>;
+        case 4: return k_shadow<256, 32, Mode>;
+        case 5: return k_shadow<256, 64, Mode>;
+        default: return k_shadow<128, 64, Mode>;
     }
 }
+inline ExtendKernel extend_kernel(int mode, int k) {
+    if (mode == kTraceBinary) return k_extend<128, 64, kTraceBinary>;
+    if (mode == kTraceWide) return k == 6 ? k_extend<128, kDeepStack, kTraceWide> : extend_shape<kTraceWide>(k);
+    return k == 6 ? k_extend<128, kDeepStack, kTraceWideWatertight> : k_extend<128, 64, kTraceWideWatertight>;
+}
+inline ShadowKernel shadow_kernel(int mode, int k) {
+    if (mode == kTraceBinary) return k_shadow<128, 64, kTraceBinary>;
+    if (mode == kTraceWide) return k == 6 ? k_shadow<128, kDeepStack, kTraceWide> : shadow_shape<kTraceWide>(k);
+    return k == 6 ? k_shadow<128, kDeepStack, kTraceWideWatertight> : k_shadow<128, 64, kTraceWideWatertight>;
+}
+inline int trace_block(int mode, int k) { return mode == kTraceWide ? trace_shape_block(k) : 128; }
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -1187,7 +1215,7 @@ struct Wavefront {
     // launch shapes
     int sms = 0;
     int grid_raygen = 0, grid_shade = 0, grid_finalize = 0;
-    int grid_extend[6] = {}, grid_shadow[6] = {};   // per traversal shape (trace_shape_index)
+    int grid_extend[kTraceModes][kTraceShapes] = {}, grid_shadow[kTraceModes][kTraceShapes] = {};
     // stats
     unsigned long long host_stats[kStatCount] = {};
     double stage_ms[5] = {0, 0, 0, 0, 0};   // extend, shade, shadow, other, guide
@@ -1253,10 +1281,11 @@ int wavefront_prepare(Wavefront& wf, int device, int npath, int n_slots) {
         wf.sms = sms;
         wf.grid_raygen = grid_for(reinterpret_cast<const void*>(k_raygen), 256, sms);
         wf.grid_shade = grid_for(reinterpret_cast<const void*>(k_shade_front<false>), 128, sms);
-        for (int k = 0; k < 6; ++k) {
-            wf.grid_extend[k] = grid_for(extend_kernel(k), trace_shape_block(k), sms);
-            wf.grid_shadow[k] = grid_for(shadow_kernel(k), trace_shape_block(k), sms);
-        }
+        for (int m = 0; m < kTraceModes; ++m)
+            for (int k = 0; k < kTraceShapes; ++k) {
+                wf.grid_extend[m][k] = grid_for(reinterpret_cast<const void*>(extend_kernel(m, k)), trace_block(m, k), sms);
+                wf.grid_shadow[m][k] = grid_for(reinterpret_cast<const void*>(shadow_kernel(m, k)), trace_block(m, k), sms);
+            }
         wf.grid_finalize = grid_for(reinterpret_cast<const void*>(k_finalize), 256, sms);
         wf.device = device;
         wf.npath = 0;
@@ -1358,12 +1387,18 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
     const int lanes = std::max(1, P.npath / std::max(P.npix, 1));
     const int total = static_cast<int>(total_samples);
     const int tsi = trace_shape_index(P.trace_block, P.stack_depth);
+    // the counters count the reference's binary walk
+    const int walk = !P.scene.wide_on || (P.flags & PT_FLAG_COUNT_TRAVERSAL) ? kTraceBinary
+                     : (P.flags & PT_FLAG_WATERTIGHT)                        ? kTraceWideWatertight
+                                                                             : kTraceWide;
     for (int s0 = 0; s0 < total; s0 += lanes) {
         const int count = std::min(lanes, total - s0);
         if (int rc = timed(3, [&] { k_raygen<<<wf.grid_raygen, 256, 0, st>>>(P, s0, count); })) return rc;
         for (int d = 0; d < P.max_depth; ++d) {
             const int q = d & 1;
-            if (int rc = timed(0, [&] { launch_extend(tsi, wf.grid_extend[tsi], st, P, q, d); })) return rc;
+            if (int rc = timed(0, [&] {
+                    extend_kernel(walk, tsi)<<<wf.grid_extend[walk][tsi], trace_block(walk, tsi), 0, st>>>(P, q, d);
+                })) return rc;
             if (infer) {
                 if (int rc = timed(4, [&] { launch_guide_infer(*gs, P, q, wf.sms, st); })) return rc;
             }
@@ -1386,7 +1421,9 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
                         }
                     }
                 })) return rc;
-            if (int rc = timed(2, [&] { launch_shadow(tsi, wf.grid_shadow[tsi], st, P, d); })) return rc;
+            if (int rc = timed(2, [&] {
+                    shadow_kernel(walk, tsi)<<<wf.grid_shadow[walk][tsi], trace_block(walk, tsi), 0, st>>>(P);
+                })) return rc;
         }
         if (int rc = timed(3, [&] { k_finalize<<<wf.grid_finalize, 256, 0, st>>>(P, s0, count); })) return rc;
         if (train) {
@@ -1423,6 +1460,12 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
 
 }  // namespace
 
+}  // namespace ptb
+
+#include "wide_build.cuh"
+
+namespace ptb {
+
 DeviceScene device_view(const pt_scene* s) {
     DeviceScene v;
     std::memset(&v, 0, sizeof(v));
@@ -1451,6 +1494,11 @@ DeviceScene device_view(const pt_scene* s) {
     v.num_punctual = static_cast<uint32_t>(s->host.punctual.size());
     v.textures = static_cast<const unsigned long long*>(d.tex_table);
     v.num_textures = d.tex_table ? static_cast<uint32_t>(d.tex_objs.size()) : 0u;
+    v.wide_on = d.wide_on ? 1u : 0u;
+    v.wide_root = d.wide_root;
+    for (int a = 0; a < 3; ++a) v.coord_max[a] = d.coord_max[a];
+    v.wide = static_cast<const WideNode*>(d.wide);
+    v.wtris = static_cast<const WideTri*>(d.wtris);
     return v;
 }
 
@@ -1463,7 +1511,7 @@ void free_scene_device(pt_scene* s) {
     for (void* a : d.tex_arrays) if (a) cudaFreeArray(static_cast<cudaArray_t>(a));
     if (d.tex_table) cudaFree(d.tex_table);
     void* bufs[] = {d.inner, d.tris, d.vertices, d.faces, d.materials, d.emissive, d.tri_pmf,
-                    d.tri_alias, d.env_pmf, d.env_alias, d.punctual};
+                    d.tri_alias, d.env_pmf, d.env_alias, d.punctual, d.wide, d.wtris};
     for (void* b : bufs) if (b) cudaFree(b);
     d = DeviceSceneBuffers{};
 }
@@ -1590,7 +1638,7 @@ int upload_scene(pt_scene* s, int device) {
             PT_CU(cudaMemcpy2DToArray(static_cast<cudaArray_t>(d.tex_arrays[i]), 0, 0, t.rgba.data(), pitch, pitch,
                                       t.height, cudaMemcpyHostToDevice));
         }
-        return PT_OK;
+        return build_wide(ts, static_cast<uint32_t>(hs.faces.size()), d);
     }
     free_scene_device(s);
     if (int rc = ensure_device(device)) return rc;
@@ -1650,6 +1698,8 @@ int upload_scene(pt_scene* s, int device) {
         d.bytes += static_cast<uint64_t>(h.env_w) * h.env_h * 16;
     }
     if (int rc2 = upload_textures(h, d)) return rc2;
+    if (int rc2 = build_wide(t, static_cast<uint32_t>(h.faces.size()), d)) return rc2;
+    d.bytes += d.wide_bytes + d.wtris_bytes;
     d.uploaded = true;
     return PT_OK;
 }
@@ -1781,6 +1831,9 @@ int prepare_wave(pt_integrator* integ, pt_film* film, pt_scene* s, const pt_scen
     P.trace_block = rs.trace_block ? rs.trace_block : 128;
     P.stack_depth = rs.stack_depth ? rs.stack_depth : kStackDepth;
     if (P.stack_depth <= static_cast<int>(s->tables.bvh_depth)) P.stack_depth = kStackDepth;
+    // (the four-wide walk defers up to three children a level)
+    if (s->dev.wide_on && P.stack_depth < static_cast<int>(s->dev.wide_need))
+        P.stack_depth = s->dev.wide_need <= static_cast<uint32_t>(kStackDepth) ? kStackDepth : kDeepStack;
     lanes_out = lanes;
     return PT_OK;
 }
@@ -1922,6 +1975,19 @@ int integrator_reset_stats(pt_integrator* integ) {
 }
 
 // ---- diagnostics ----
+using TraceKernel = void (*)(DeviceScene, const float*, uint32_t, pt_hit*, uint8_t*, int, uint32_t*);
+template <int Depth>
+TraceKernel trace_rays_depth(bool watertight, bool any) {
+    if (watertight)
+        return any ? k_trace_rays<Depth, kTraceWideWatertight, true> : k_trace_rays<Depth, kTraceWideWatertight, false>;
+    return any ? k_trace_rays<Depth, kTraceWide, true> : k_trace_rays<Depth, kTraceWide, false>;
+}
+static TraceKernel trace_rays_kernel(const DeviceSceneBuffers& d, bool watertight, bool any) {
+    if (!d.wide_on) return any ? k_trace_rays<kStackDepth, kTraceBinary, true> : k_trace_rays<kStackDepth, kTraceBinary, false>;
+    return d.wide_need <= static_cast<uint32_t>(kStackDepth) ? trace_rays_depth<kStackDepth>(watertight, any)
+                                                             : trace_rays_depth<kDeepStack>(watertight, any);
+}
+
 int trace_rays(pt_scene* s, const float* rays, uint32_t n, pt_hit* hits, uint8_t* occl, bool any, bool device_ptrs) {
     if (!s->dev.uploaded) { set_error("scene not uploaded"); return PT_ERR_STATE; }
     if (int rc = ensure_device(s->dev.device)) return rc;
@@ -1949,9 +2015,11 @@ int trace_rays(pt_scene* s, const float* rays, uint32_t n, pt_hit* hits, uint8_t
     }
     const DeviceScene v = device_view(s);
     const int wt = (s->host.settings.flags & PT_FLAG_WATERTIGHT) ? 1 : 0;
-    const int blocks = static_cast<int>(std::min<uint32_t>((n + 127) / 128, 148u * 16u));
-    k_trace_rays<<<blocks, 128>>>(v, d_rays, n, any ? nullptr : static_cast<pt_hit*>(d_out),
-                                  any ? static_cast<uint8_t*>(d_out) : nullptr, any ? 1 : 0, wt, d_err);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev.device);
+    const int blocks = static_cast<int>(std::min<uint32_t>((n + 127) / 128, static_cast<uint32_t>(sms) * 8u));
+    trace_rays_kernel(s->dev, wt != 0, any)<<<blocks, 128>>>(v, d_rays, n, any ? nullptr : static_cast<pt_hit*>(d_out),
+                                                             any ? static_cast<uint8_t*>(d_out) : nullptr, wt, d_err);
     cudaError_t e = cudaDeviceSynchronize();
     uint32_t err = 0;
     if (e == cudaSuccess) e = cudaMemcpy(&err, d_err, 4, cudaMemcpyDeviceToHost);

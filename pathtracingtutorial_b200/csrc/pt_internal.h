@@ -163,6 +163,8 @@ static_assert(sizeof(TriRecord) == 48, "TriRecord must be 48 bytes");
 // Device scene view (DeviceSceneView + DeviceLightView,
 // Part_2/src/scene/device_scene.h:29-67), passed by value.
 // ---------------------------------------------------------------------------
+struct WideNode;   // wide.h
+struct WideTri;
 struct DeviceScene {
     const InnerNode*  inner;
     const TriRecord*  tris;
@@ -191,6 +193,12 @@ struct DeviceScene {
     // material textures (float4, bilinear, normalized coordinates)
     const unsigned long long* textures;     // cudaTextureObject_t per texture (0 = no image)
     uint32_t               num_textures;
+    // four-wide tree (wide.h)
+    uint32_t               wide_on;         // 0: rays take the binary walk
+    uint32_t               wide_root;       // 0, or kLeafBit|first for a one-leaf tree
+    float                  coord_max[3];    // largest |coordinate| per axis
+    const WideNode*        wide;
+    const WideTri*         wtris;
 };
 
 // Ray as stored in queues: origin (w unused) and direction (w = tmax for shadow rays).
