@@ -110,8 +110,9 @@ PT_HD f3 sample_vndf(f3 wo, float ax, float ay, float u1, float u2) {
     const f3 t2v = cross(wh, t1v);
     const float r = sqrtf(u1);
     const float phi = kTwoPi * u2;
-    const float p1 = r * cosf(phi);
-    float p2 = r * sinf(phi);
+    const float2 cs = cos_sin(phi);
+    const float p1 = r * cs.x;
+    float p2 = r * cs.y;
     const float s = 0.5f * (1.0f + wh.z);
     p2 = (1.0f - s) * sqrtf(fmaxf(0.0f, 1.0f - p1 * p1)) + s * p2;
     const f3 nh = p1 * t1v + p2 * t2v + sqrtf(fmaxf(0.0f, 1.0f - p1 * p1 - p2 * p2)) * wh;
@@ -146,13 +147,13 @@ PT_HD f3 tint_of(f3 base) {
 }
 PT_HD f3 disney_diffuse(const MatEval& m, float nol, float nov, float hol) {
     const float fd90 = 0.5f + 2.0f * hol * hol * m.roughness;
-    const float fl = 1.0f + (fd90 - 1.0f) * powf(1.0f - nol, 5.0f);
-    const float fv = 1.0f + (fd90 - 1.0f) * powf(1.0f - nov, 5.0f);
+    const float fl = 1.0f + (fd90 - 1.0f) * pow_5(1.0f - nol);
+    const float fv = 1.0f + (fd90 - 1.0f) * pow_5(1.0f - nov);
     f3 d = m.base * (kInvPi * fl * fv);
     if (m.subsurface > 0.0f) {
         const float fss90 = hol * hol * m.roughness;
-        const float sl = 1.0f + (fss90 - 1.0f) * powf(1.0f - nol, 5.0f);
-        const float sv = 1.0f + (fss90 - 1.0f) * powf(1.0f - nov, 5.0f);
+        const float sl = 1.0f + (fss90 - 1.0f) * pow_5(1.0f - nol);
+        const float sv = 1.0f + (fss90 - 1.0f) * pow_5(1.0f - nov);
         const float ss = 1.25f * (sl * sv * (1.0f / (nol + nov + 1e-5f) - 0.5f) + 0.5f);
         d = (1.0f - m.subsurface) * d + m.subsurface * (m.base * (kInvPi * ss));
     }
@@ -161,7 +162,7 @@ PT_HD f3 disney_diffuse(const MatEval& m, float nol, float nov, float hol) {
 PT_HD f3 disney_sheen(const MatEval& m, float hol) {
     if (m.sheen <= 0.0f) return mk(0.0f);
     const f3 c = ((1.0f - m.sheen_tint) * mk(1.0f) + m.sheen_tint * tint_of(m.base)) * m.sheen_color;
-    return m.sheen * c * powf(1.0f - hol, 5.0f);
+    return m.sheen * c * pow_5(1.0f - hol);
 }
 PT_HD f3 disney_f0(const MatEval& m) {
     const float eta = m.ior;
@@ -314,7 +315,8 @@ PT_HD bool disney_sample_dir(const MatEval& m, f3 wo, f3 n, PathRng& rng, int rt
         // cosine hemisphere (Malley)
         const float rr = sqrtf(u1);
         const float phi = kTwoPi * u2;
-        wi = to_world(fr, mk(rr * cosf(phi), rr * sinf(phi), sqrtf(fmaxf(0.0f, 1.0f - u1))));
+        const float2 cs = cos_sin(phi);
+        wi = to_world(fr, mk(rr * cs.x, rr * cs.y, sqrtf(fmaxf(0.0f, 1.0f - u1))));
     } else if (choice < w.diff + w.sheen + w.spec) {
         const f3 h = to_world(fr, sample_vndf(wol, ax, ay, u1, u2));
         wi = reflect(-wo, h);

@@ -169,7 +169,7 @@ __device__ __forceinline__ float4 tex_at(const DeviceScene& s, int32_t id, float
     return tex2D<float4>(static_cast<cudaTextureObject_t>(s.textures[id]), u, v);
 }
 // texel colour to linear (the reference's pow(c, 2.2) per channel)
-__device__ __forceinline__ f3 tex_linear(float4 c) { return mk(powf(c.x, 2.2f), powf(c.y, 2.2f), powf(c.z, 2.2f)); }
+__device__ __forceinline__ f3 tex_linear(float4 c) { return mk(pow_2_2(c.x), pow_2_2(c.y), pow_2_2(c.z)); }
 __device__ __forceinline__ float2 vuv(const DeviceScene& s, uint32_t i) {
     return __ldg(reinterpret_cast<const float2*>(s.vertices + i) + 4);
 }
@@ -329,7 +329,9 @@ __global__ void k_begin(PassState* ps, uint32_t frame) { ps->frame = frame; }
 __device__ __forceinline__ PathRng make_rng(int type, int x, int y, uint32_t frame, uint32_t spf, uint32_t i,
                                             uint32_t user_seed) {
     PathRng rng;
-    rng.type = type; rng.px = x; rng.py = y; rng.sample_index = frame * spf + i;
+    rng.type = type;
+    rng.pixel = type == PT_SAMPLER_SOBOL ? pixel_hash(x, y) : 0u;
+    rng.rev_index = bit_reverse(frame * spf + i);
     rng.s = (type == PT_SAMPLER_SOBOL) ? 0u : pcg_seed(x, y, frame, i, user_seed);
     return rng;
 }
@@ -772,10 +774,13 @@ __device__ bool shade_path(const DeviceScene& s, int arg_rtl, int depth, bool la
 __device__ __forceinline__ PathRng path_rng(const WaveParams& P, uint32_t p, uint32_t sidx0) {
     PathRng rng;
     rng.type = P.sampler_type;
-    const uint32_t pix = p % static_cast<uint32_t>(P.npix);
-    rng.px = static_cast<int>(pix % static_cast<uint32_t>(P.width));
-    rng.py = static_cast<int>(pix / static_cast<uint32_t>(P.width));
-    rng.sample_index = sidx0 + p / static_cast<uint32_t>(P.npix);
+    rng.pixel = rng.rev_index = 0u;
+    if (P.sampler_type == PT_SAMPLER_SOBOL) {
+        const uint32_t pix = p % static_cast<uint32_t>(P.npix);
+        rng.pixel = pixel_hash(static_cast<int>(pix % static_cast<uint32_t>(P.width)),
+                               static_cast<int>(pix / static_cast<uint32_t>(P.width)));
+        rng.rev_index = bit_reverse(sidx0 + p / static_cast<uint32_t>(P.npix));
+    }
     rng.s = P.rng[p];
     return rng;
 }
@@ -801,20 +806,78 @@ __device__ __forceinline__ void push_continuation(const WaveParams& P, int q, bo
 // cache less (on the 1080p bench render: shading 325 -> 243 ms); the front
 // hands the shading point to the back in the queue entry's own slots:
 // hit[i] = (point, prim | entering << 30, or -1 when the path needs no
-// sampling), ray_o[q][i] = (geometric normal, roulette weight).  Both run 6
-// blocks of 128 per SM (80 registers): 224 ms against 243 ms at 5 blocks.
+// sampling), ray_o[q][i] = (geometric normal, roulette weight).  Both hold 24
+// warps per SM (80 registers).
+//
+// They wait for instructions more than for anything else: the code is 66 to
+// 110 KB, and warps at different places in it evict one another's lines.  So
+// the warps of a block start every queue entry together (a barrier a tile),
+// in blocks of 256, and of 768 -- the whole SM in step -- for the textured
+// kernels, whose code is the longest.  Shading stage, blocks of 128 without
+// the barrier -> this: Cornell box 512 x 512, 64 spp 10.1 -> 9.7 ms; textured
+// Cornell box 803 x 601, 32 spp 18.4 -> 12.8 ms (256: 14.3, 384: 13.6); closed
+// room 1024 x 1024, 64 spp 73 -> 71 ms (768: 75).
+constexpr int shade_block(bool textured) { return textured ? 768 : 256; }
+constexpr int kShadeThreads = 768;   // per SM
 constexpr uint32_t kEnteringBit = 0x40000000u;
 
-template <bool Guided, bool Textured = false>
-__global__ void __launch_bounds__(128, 6) k_shade_front(WaveParams P, int q, int depth, int s0) {
+// Splits a block's share of a queue into hits and misses: tiles are read into
+// two rings until one holds an entry for every thread, which is then the next
+// batch; the last ones are smaller.  All threads call it.  B: block size.
+template <int B>
+struct HitMissFeed {
+    uint32_t list[2][2 * B], count[2], head[2];
+    // entry for this thread (0xffffffff: none); false when the queue is done
+    __device__ __forceinline__ bool next(const float4* hit, uint32_t& tile, uint32_t n, uint32_t& entry) {
+        auto wrap = [](uint32_t x) { return x >= 2u * B ? x - 2u * B : x; };
+        while (tile < n && count[0] < B && count[1] < B) {
+            const uint32_t e = tile + threadIdx.x;
+            tile += gridDim.x * B;
+            __syncthreads();   // every thread has read the counts
+            const bool have = e < n;
+            const bool miss = have && __float_as_int(hit[e].y) < 0;
+            const uint32_t mh = __ballot_sync(0xffffffffu, have && !miss), mm = __ballot_sync(0xffffffffu, miss);
+            const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+            uint32_t b0 = 0, b1 = 0;
+            if (lane == 0) {
+                b0 = atomicAdd(&count[0], static_cast<uint32_t>(__popc(mh)));
+                b1 = atomicAdd(&count[1], static_cast<uint32_t>(__popc(mm)));
+            }
+            b0 = __shfl_sync(0xffffffffu, b0, 0);
+            b1 = __shfl_sync(0xffffffffu, b1, 0);
+            if (miss) list[1][wrap(head[1] + b1 + __popc(mm & below))] = e;
+            else if (have) list[0][wrap(head[0] + b0 + __popc(mh & below))] = e;
+            __syncthreads();
+        }
+        const uint32_t which = count[0] >= B ? 0u : (count[1] >= B ? 1u : (count[0] ? 0u : 1u));
+        const uint32_t c = count[which], take = min(c, static_cast<uint32_t>(B));
+        entry = threadIdx.x < take ? list[which][wrap(head[which] + threadIdx.x)] : 0xffffffffu;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            count[which] = c - take;
+            head[which] = wrap(head[which] + take);
+        }
+        __syncthreads();
+        return c != 0u;
+    }
+};
+
+// Split: batches of hits and of misses (HitMissFeed).  Under an open sky half
+// or more of a bounce's rays escape, which left 10.8 of 32 lanes active in the
+// second bounce of the 2M-triangle field: its shading stage 3.4 -> 3.06 ms at
+// full HD, 4 spp.  Without an environment few rays escape, and the split only
+// costs (closed room 71 -> 72.5 ms).
+template <bool Guided, bool Textured, bool Split>
+__global__ void __launch_bounds__(shade_block(Textured), kShadeThreads / shade_block(Textured))
+k_shade_front(WaveParams P, int q, int depth, int s0) {
     const uint32_t cap = static_cast<uint32_t>(P.npath);
     const uint32_t n = min(P.counts[q], cap);
     const uint32_t sidx0 = P.pass->frame * static_cast<uint32_t>(P.spf) + static_cast<uint32_t>(s0);
     const bool last = depth == P.max_depth - 1;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    constexpr int B = shade_block(Textured);
+    auto shade = [&](const uint32_t i) {
         const uint32_t p = P.queue[q][i];
-        if (p >= cap) { atomicOr(P.err, kErrQueueOverflow); continue; }
+        if (p >= cap) { atomicOr(P.err, kErrQueueOverflow); return; }
         const float4 o4 = P.ray_o[q][i];
         const float4 d4 = P.ray_d[q][i];
         const float4 h = P.hit[i];
@@ -862,17 +925,34 @@ __global__ void __launch_bounds__(128, 6) k_shade_front(WaveParams P, int q, int
             P.hit[i].w = __int_as_float(-1);
         }
         push_continuation(P, q, r == 2 && !last, p, no, nd, Guided ? o4.w : 1.0f);
+    };
+    uint32_t tile = blockIdx.x * B;
+    if constexpr (Split) {
+        __shared__ HitMissFeed<B> feed;
+        if (threadIdx.x < 2) feed.count[threadIdx.x] = feed.head[threadIdx.x] = 0u;
+        __syncthreads();
+        uint32_t i;
+        while (feed.next(P.hit, tile, n, i))
+            if (i != 0xffffffffu) shade(i);
+    } else {
+        for (; tile < n; tile += gridDim.x * B) {
+            __syncthreads();
+            if (tile + threadIdx.x < n) shade(tile + threadIdx.x);
+        }
     }
 }
 
-template <bool Guided, bool Textured = false>
-__global__ void __launch_bounds__(128, 6) k_shade_back(WaveParams P, int q, int depth, int s0) {
+template <bool Guided, bool Textured>
+__global__ void __launch_bounds__(shade_block(Textured), kShadeThreads / shade_block(Textured))
+k_shade_back(WaveParams P, int q, int depth, int s0) {
     const uint32_t cap = static_cast<uint32_t>(P.npath);
     const uint32_t n = min(P.counts[4], cap);
     const uint32_t sidx0 = P.pass->frame * static_cast<uint32_t>(P.spf) + static_cast<uint32_t>(s0);
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
-        const uint32_t i = P.slist[j];
+    for (uint32_t tile = blockIdx.x * blockDim.x; tile < n; tile += stride) {
+        __syncthreads();
+        if (tile + threadIdx.x >= n) continue;
+        const uint32_t i = P.slist[tile + threadIdx.x];
         const float4 h = P.hit[i];
         const int code = Textured ? __float_as_int(h.y) : __float_as_int(h.w);
         bool cont = false;
@@ -1128,10 +1208,7 @@ __global__ void k_sampler_stream(int type, int w, int h, uint32_t frame, int spf
                                  uint32_t seed, float* out) {
     const int npix = w * h;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
-        PathRng r;
-        r.type = type; r.px = p % w; r.py = p / w;
-        r.sample_index = frame * static_cast<uint32_t>(spf) + static_cast<uint32_t>(sif);
-        r.s = type == PT_SAMPLER_SOBOL ? 0u : pcg_seed(r.px, r.py, frame, static_cast<uint32_t>(sif), seed);
+        PathRng r = make_rng(type, p % w, p / w, frame, static_cast<uint32_t>(spf), static_cast<uint32_t>(sif), seed);
         for (uint32_t k = 0; k < ndims; ++k) out[static_cast<size_t>(p) * ndims + k] = rng_next(r);
     }
 }
@@ -1158,6 +1235,20 @@ inline int trace_shape_index(int block, int depth) {
     return (block == 64 ? 0 : (block == 256 ? 2 : 1)) * 2 + (depth == 32 ? 0 : 1);
 }
 inline int trace_shape_block(int k) { return k == 6 ? 128 : (k < 2 ? 64 : (k < 4 ? 128 : 256)); }
+
+using ShadeKernel = void (*)(WaveParams, int, int, int);
+inline ShadeKernel shade_front_kernel(bool guided, bool textured, bool split) {
+    if (guided) {
+        if (textured) return split ? k_shade_front<true, true, true> : k_shade_front<true, true, false>;
+        return split ? k_shade_front<true, false, true> : k_shade_front<true, false, false>;
+    }
+    if (textured) return split ? k_shade_front<false, true, true> : k_shade_front<false, true, false>;
+    return split ? k_shade_front<false, false, true> : k_shade_front<false, false, false>;
+}
+inline ShadeKernel shade_back_kernel(bool guided, bool textured) {
+    if (guided) return textured ? k_shade_back<true, true> : k_shade_back<true, false>;
+    return textured ? k_shade_back<false, true> : k_shade_back<false, false>;
+}
 
 using ExtendKernel = void (*)(WaveParams, int, int);
 using ShadowKernel = void (*)(WaveParams);
@@ -1214,7 +1305,7 @@ struct Wavefront {
     cudaStream_t graph_stream = nullptr;
     // launch shapes
     int sms = 0;
-    int grid_raygen = 0, grid_shade = 0, grid_finalize = 0;
+    int grid_raygen = 0, grid_finalize = 0;
     int grid_extend[kTraceModes][kTraceShapes] = {}, grid_shadow[kTraceModes][kTraceShapes] = {};
     // stats
     unsigned long long host_stats[kStatCount] = {};
@@ -1280,7 +1371,6 @@ int wavefront_prepare(Wavefront& wf, int device, int npath, int n_slots) {
         PT_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         wf.sms = sms;
         wf.grid_raygen = grid_for(reinterpret_cast<const void*>(k_raygen), 256, sms);
-        wf.grid_shade = grid_for(reinterpret_cast<const void*>(k_shade_front<false>), 128, sms);
         for (int m = 0; m < kTraceModes; ++m)
             for (int k = 0; k < kTraceShapes; ++k) {
                 wf.grid_extend[m][k] = grid_for(reinterpret_cast<const void*>(extend_kernel(m, k)), trace_block(m, k), sms);
@@ -1403,23 +1493,10 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
                 if (int rc = timed(4, [&] { launch_guide_infer(*gs, P, q, wf.sms, st); })) return rc;
             }
             if (int rc = timed(1, [&] {
-                    const bool tex = P.scene.num_textures > 0;
-                    if (P.gmix) {
-                        if (tex) k_shade_front<true, true><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                        else k_shade_front<true><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                    } else {
-                        if (tex) k_shade_front<false, true><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                        else k_shade_front<false><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                    }
-                    if (d + 1 < P.max_depth) {
-                        if (P.gmix) {
-                            if (tex) k_shade_back<true, true><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                            else k_shade_back<true><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                        } else {
-                            if (tex) k_shade_back<false, true><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                            else k_shade_back<false><<<wf.grid_shade, 128, 0, st>>>(P, q, d, s0);
-                        }
-                    }
+                    const bool tex = P.scene.num_textures > 0, guided = P.gmix != nullptr;
+                    const int b = shade_block(tex), grid = wf.sms * (kShadeThreads / b);
+                    shade_front_kernel(guided, tex, P.scene.env_tex != 0)<<<grid, b, 0, st>>>(P, q, d, s0);
+                    if (d + 1 < P.max_depth) shade_back_kernel(guided, tex)<<<grid, b, 0, st>>>(P, q, d, s0);
                 })) return rc;
             if (int rc = timed(2, [&] {
                     shadow_kernel(walk, tsi)<<<wf.grid_shadow[walk][tsi], trace_block(walk, tsi), 0, st>>>(P);

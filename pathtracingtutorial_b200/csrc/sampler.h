@@ -49,12 +49,14 @@ PT_HD uint32_t lk_hash(uint32_t x, uint32_t seed) {
     return x;
 }
 
-PT_HD uint32_t pixel_dim_seed(int px, int py, uint32_t dim) {
+// The pixel's part of the dimension hash, and the dimension's.
+PT_HD uint32_t pixel_hash(int px, int py) {
     uint32_t h = mix32(static_cast<uint32_t>(px) + 0x9e3779b9u);
     h ^= static_cast<uint32_t>(py) + 0x9e3779b9u + (h << 6) + (h >> 2);
-    h = mix32(h);
-    h ^= dim + 0x9e3779b9u + (h << 6) + (h >> 2);
     return mix32(h);
+}
+PT_HD uint32_t dim_seed(uint32_t pixel, uint32_t dim) {
+    return mix32(pixel ^ (dim + 0x9e3779b9u + (pixel << 6) + (pixel >> 2)));
 }
 
 PT_HD float u32_to_unit(uint32_t v) {
@@ -62,10 +64,11 @@ PT_HD float u32_to_unit(uint32_t v) {
     return static_cast<float>(v) * 2.3283064365386963e-10f;
 }
 
-// One Sobol draw: dimension `dim` of sample `sample_index` for pixel (px, py).
-PT_HD float sobol_draw(int px, int py, uint32_t sample_index, uint32_t dim) {
-    const uint32_t seed = pixel_dim_seed(px, py, dim);
-    const uint32_t shuffled = bit_reverse(lk_hash(bit_reverse(sample_index), seed));
+// One Sobol draw: dimension `dim` of the sample with the bit-reversed index
+// rev_index for the pixel with this pixel_hash.
+PT_HD float sobol_draw(uint32_t pixel, uint32_t rev_index, uint32_t dim) {
+    const uint32_t seed = dim_seed(pixel, dim);
+    const uint32_t shuffled = bit_reverse(lk_hash(rev_index, seed));
     const uint32_t value = bit_reverse(lk_hash(shuffled, mix32(seed)));
     return fminf(u32_to_unit(value), 0.99999994f);
 }
@@ -86,17 +89,19 @@ PT_HD float pcg_draw(uint32_t& state) {
 }
 
 // Per-path sampler state.  For Sobol `s` is the next dimension; for PCG it is
-// the generator state.
+// the generator state.  The pixel's half of the Sobol hash and the reversed
+// sample index are the same for all of a path's draws, so they are made once
+// (a draw is two hash rounds shorter for it); PCG uses neither.
 struct PathRng {
     int      type;
-    int      px, py;
-    uint32_t sample_index;
+    uint32_t pixel;       // pixel_hash(px, py)
+    uint32_t rev_index;   // bit-reversed sample index
     uint32_t s;
 };
 
 PT_HD float rng_next(PathRng& r) {
     if (r.type == PT_SAMPLER_SOBOL) {
-        float v = sobol_draw(r.px, r.py, r.sample_index, r.s);
+        float v = sobol_draw(r.pixel, r.rev_index, r.s);
         r.s += 1u;
         return v;
     }
