@@ -355,7 +355,7 @@ int batch_wavefront(const pt_batch_item* in, uint32_t n, int out_is_device, int6
         cudaStream_t bs = (*side)[k % branches];
         Wavefront& wf = *slots[k]->integ->wf;
         k_begin<<<1, 1, 0, bs>>>(P[k].pass, in[k].first_frame);
-        rc = enqueue_batch(wf, P[k], total[k], bs, nullptr, wf.guide);
+        rc = enqueue_batch(wf, P[k], total[k], bs, nullptr, wf.guide, false);
         if (rc == PT_OK && write_out) {
             const int np = P[k].npix;
             float4* out = out_is_device ? reinterpret_cast<float4*>(in[k].out_rgba)
