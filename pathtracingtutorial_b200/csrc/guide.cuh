@@ -258,13 +258,16 @@ __device__ __forceinline__ void encode_a(const GuideNet& net, f3 p0, f3 p1, uint
     }
 }
 
+// Weights into shared memory, 16 bytes a copy (rows are 64 or 128 bytes, their
+// padded places 80 or 144 bytes apart).
 __device__ __forceinline__ void load_weights_smem(const GuideNet& net, __nv_bfloat16* sw) {
+#pragma unroll
     for (int l = 0; l < 4; ++l) {
-        const int in = g_in(l), out = g_out(l), ld = g_sld(l);
-        for (int i = threadIdx.x; i < out * in; i += blockDim.x) {
-            const int o = i / in, k = i % in;
-            sw[g_soff(l) + o * ld + k] = net.w[g_woff(l) + i];
-        }
+        constexpr int kPer = 8;   // elements a copy
+        const int per_row = g_in(l) / kPer;
+        const uint4* src = reinterpret_cast<const uint4*>(net.w + g_woff(l));
+        for (int i = threadIdx.x; i < g_out(l) * per_row; i += blockDim.x)
+            *reinterpret_cast<uint4*>(sw + g_soff(l) + (i / per_row) * g_sld(l) + (i % per_row) * kPer) = src[i];
     }
     __syncthreads();
 }
@@ -294,6 +297,7 @@ __device__ __forceinline__ void raw_to_mixture(const float* raw, float* mix) {
     float mx = -1e30f;
     for (int k = 0; k < kGLobes; ++k) mx = fmaxf(mx, raw[5 * k + 4]);
     float sum = 0.0f;
+#pragma unroll 1
     for (int k = 0; k < kGLobes; ++k) {
         f3 m = mk(raw[5 * k], raw[5 * k + 1], raw[5 * k + 2]);
         const float l = length(m);
@@ -457,6 +461,7 @@ __device__ float mixture_grad(const float* raw, f3 dir, float w, float* d) {
     raw_to_mixture(raw, mix);
     float v[kGLobes];
     float q = 0.0f;
+#pragma unroll 1
     for (int k = 0; k < kGLobes; ++k) {
         const float c = mix[4 * k] * dir.x + mix[4 * k + 1] * dir.y + mix[4 * k + 2] * dir.z;
         v[k] = vmf_pdf(mix[4 * k + 3], c);
@@ -464,6 +469,7 @@ __device__ float mixture_grad(const float* raw, f3 dir, float w, float* d) {
     }
     q = fmaxf(q, 1e-12f);
     const float gq = -w / q;
+#pragma unroll 1
     for (int k = 0; k < kGLobes; ++k) {
         const float pi = mix[32 + k], kap = mix[4 * k + 3];
         const f3 mu = mk(mix[4 * k], mix[4 * k + 1], mix[4 * k + 2]);
@@ -638,14 +644,19 @@ __global__ void __launch_bounds__(32 * kGTrainWarps) k_guide_train(GuideNet net,
     __nv_bfloat16* swt = sw + kGSmemW;                                                 // WT [in][out+8]
     unsigned char* scratch0 = reinterpret_cast<unsigned char*>(swt + kGSmemW + 64);
     load_weights_smem(net, sw);
-    // transposed weights: layer l, WT[in][out] with row length out + 8
+    // transposed weights: layer l, WT[in][out] with row length out + 8, from the
+    // copy in shared memory, two outputs a store
+#pragma unroll
     for (int l = 0; l < 4; ++l) {
-        const int in = g_in(l), out = g_out(l);
+        const int in = g_in(l), out = g_out(l), ld = g_sld(l);
         const int woff = l == 0 ? 0 : (l == 1 ? kGIn * (kGHid + 8) : (l == 2 ? kGIn * (kGHid + 8) + kGHid * (kGHid + 8)
                                                                              : kGIn * (kGHid + 8) + 2 * kGHid * (kGHid + 8)));
-        for (int i = threadIdx.x; i < out * in; i += blockDim.x) {
-            const int o = i / in, k = i % in;
-            swt[woff + k * (out + 8) + o] = net.w[g_woff(l) + i];
+        for (int i = threadIdx.x; i < out / 2 * in; i += blockDim.x) {
+            const int k = i % in, o = i / in * 2;
+            __nv_bfloat162 v;
+            v.x = sw[g_soff(l) + o * ld + k];
+            v.y = sw[g_soff(l) + (o + 1) * ld + k];
+            *reinterpret_cast<__nv_bfloat162*>(swt + woff + k * (out + 8) + o) = v;
         }
     }
     __syncthreads();
@@ -752,29 +763,37 @@ __global__ void __launch_bounds__(32 * kGTrainWarps) k_guide_train(GuideNet net,
         float dx[4][4];
         back_dx<kGHid, kGIn>(DY, WT0, dx);
         __syncwarp();
-        // scatter the input gradient to the hash grid (levels c, 4+c, 8+c, 12+c)
+        // Scatter the input gradient to the hash grid (through shared memory, so
+        // that the loop over the levels is one copy of its code).  Four lanes
+        // take a row, lane (corner x, feature): the four sums of a cell edge
+        // along x are 32 contiguous bytes, so an atomic instruction touches 8 to
+        // 16 sectors instead of 32.
+        constexpr int kGxLd = 2 * kGLevels + 2;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            const int level = nt * 4 + c;
+            *reinterpret_cast<float2*>(OUT + g * kGxLd + 2 * (nt * 4 + c)) = make_float2(dx[nt][0], dx[nt][1]);
+            *reinterpret_cast<float2*>(OUT + (g + 8) * kGxLd + 2 * (nt * 4 + c)) = make_float2(dx[nt][2], dx[nt][3]);
+        }
+        __syncwarp();
+        const uint32_t cx = static_cast<uint32_t>(c) >> 1, f = static_cast<uint32_t>(c) & 1u;
+#pragma unroll 1
+        for (int k = 0; k < 2 * kGLevels; ++k) {
+            const int level = k >> 1, half = k & 1;
+            if ((half ? r1 : r0) >= n) continue;
+            const f3 p = half ? p1 : p0;
+            const float gv = OUT[(g + 8 * half) * kGxLd + 2 * level + f];
+            const float sc = net.scale[level];
+            const float fx = p.x * sc + 0.5f, fy = p.y * sc + 0.5f, fz = p.z * sc + 0.5f;
+            const float bx = floorf(fx), by = floorf(fy), bz = floorf(fz);
+            const float tx = fx - bx, ty = fy - by, tz = fz - bz;
+            const uint32_t ix = static_cast<uint32_t>(bx), iy = static_cast<uint32_t>(by), iz = static_cast<uint32_t>(bz);
+            unsigned long long* gg = net.grid_grad + static_cast<size_t>(level) * kGTable * 2;
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const uint32_t r = half ? r1 : r0;
-                if (r >= n) continue;
-                const f3 p = half ? p1 : p0;
-                const float gx = dx[nt][2 * half], gy = dx[nt][2 * half + 1];
-                const float sc = net.scale[level];
-                const float fx = p.x * sc + 0.5f, fy = p.y * sc + 0.5f, fz = p.z * sc + 0.5f;
-                const float bx = floorf(fx), by = floorf(fy), bz = floorf(fz);
-                const float tx = fx - bx, ty = fy - by, tz = fz - bz;
-                const uint32_t ix = static_cast<uint32_t>(bx), iy = static_cast<uint32_t>(by), iz = static_cast<uint32_t>(bz);
-                unsigned long long* gg = net.grid_grad + static_cast<size_t>(level) * kGTable * 2;
-                for (int cidx = 0; cidx < 8; ++cidx) {
-                    const uint32_t cx = cidx & 1, cy = (cidx >> 1) & 1, cz = (cidx >> 2) & 1;
-                    const float w = (cx ? tx : 1.0f - tx) * (cy ? ty : 1.0f - ty) * (cz ? tz : 1.0f - tz);
-                    const uint32_t e = grid_index(net, level, ix + cx, iy + cy, iz + cz);
-                    atomicAdd(&gg[2 * e], g_fix(w * gx));
-                    atomicAdd(&gg[2 * e + 1], g_fix(w * gy));
-                }
+            for (uint32_t e = 0; e < 4; ++e) {
+                const uint32_t cy = e & 1, cz = e >> 1;
+                const float w = (cx ? tx : 1.0f - tx) * (cy ? ty : 1.0f - ty) * (cz ? tz : 1.0f - tz);
+                const uint32_t j = grid_index(net, level, ix + cx, iy + cy, iz + cz);
+                atomicAdd(&gg[2 * j + f], g_fix(w * gv));
             }
         }
         __syncwarp();
@@ -898,6 +917,20 @@ __global__ void k_guide_step(uint32_t* sample_count, uint32_t* step, float* loss
     loss_fix[1] = 0ull;
 }
 
+// The optimiser's running averages a x + b y with one product fused into the
+// sum -- the second for the grid and every parameter average, the first for
+// the weights' moments.  Training is chaotic: the rounding is spelled out so
+// that it does not depend on how the compiler contracts the sum.
+__device__ __forceinline__ float blend_second(float a, float x, float b, float y) { return fmaf(b, y, __fmul_rn(a, x)); }
+__device__ __forceinline__ float blend_first(float a, float x, float b, float y) { return fmaf(a, x, __fmul_rn(b, y)); }
+// b v + (1 - b) g g
+__device__ __forceinline__ float square_second(float b, float v, float g) {
+    return fmaf(__fmul_rn(1.0f - b, g), g, __fmul_rn(b, v));
+}
+__device__ __forceinline__ float square_first(float b, float v, float g) {
+    return fmaf(b, v, __fmul_rn(__fmul_rn(1.0f - b, g), g));
+}
+
 // Adam step for minibatch mb (skipped when it is empty); the step number is
 // the counter plus the non-empty minibatches before it, plus one.
 __global__ void k_guide_adam(GuideNet net, const uint32_t* count, uint32_t cap, int mb, int nmb, const uint32_t* step,
@@ -914,44 +947,72 @@ __global__ void k_guide_adam(GuideNet net, const uint32_t* count, uint32_t cap, 
     const float ea = net.ema, eb = 1.0f - net.ema;
     const size_t nw = kGWeights;
     const size_t ng = static_cast<size_t>(kGLevels) * kGTable;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < nw + ng;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        if (i < nw) {
-            const float gr = g_unfix(net.w_grad[i]);
-            const float m = b1 * net.w_m[i] + (1.0f - b1) * gr;
-            const float v = b2 * net.w_v[i] + (1.0f - b2) * gr * gr;
-            net.w_m[i] = m; net.w_v[i] = v; net.w_grad[i] = 0ull;
-            const float p = net.w_master[i] - lr_w * (m / bc1) / (sqrtf(v / bc2) + eps);
-            net.w_master[i] = p;
-            net.w[i] = __float2bfloat16_rn(p);
-            if (ea > 0.0f) {
-                const float e = ea * net.w_ema[i] + eb * p;
-                net.w_ema[i] = e;
-                net.w_inf[i] = __float2bfloat16_rn(e);
-            }
-        } else {
-            const size_t j = i - nw;
-            const ulonglong2 gi = reinterpret_cast<const ulonglong2*>(net.grid_grad)[j];
-            if (gi.x == 0ull && gi.y == 0ull && net.grid_m[j].x == 0.0f && net.grid_m[j].y == 0.0f) continue;
+    const size_t first = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+    for (size_t i = first; i < nw; i += stride) {
+        const float gr = g_unfix(net.w_grad[i]);
+        const float m = blend_first(b1, net.w_m[i], 1.0f - b1, gr);
+        const float v = square_first(b2, net.w_v[i], gr);
+        net.w_m[i] = m; net.w_v[i] = v; net.w_grad[i] = 0ull;
+        const float p = net.w_master[i] - lr_w * (m / bc1) / (sqrtf(v / bc2) + eps);
+        net.w_master[i] = p;
+        net.w[i] = __float2bfloat16_rn(p);
+        if (ea > 0.0f) {
+            const float e = blend_second(ea, net.w_ema[i], eb, p);
+            net.w_ema[i] = e;
+            net.w_inf[i] = __float2bfloat16_rn(e);
+        }
+    }
+    // The grid, two neighbouring entries a thread: all of their state is
+    // fetched at once in 16-byte loads (one entry at a time, the moments after
+    // the gradient, left the kernel waiting for memory at half its rate).
+    for (size_t k = first; k < ng / 2; k += stride) {
+        const ulonglong2* gp = reinterpret_cast<const ulonglong2*>(net.grid_grad) + 2 * k;
+        const ulonglong2 g2[2] = {gp[0], gp[1]};
+        const float4 m4 = reinterpret_cast<const float4*>(net.grid_m)[k];
+        const float4 v4 = reinterpret_cast<const float4*>(net.grid_v)[k];
+        const float4 p4 = reinterpret_cast<const float4*>(net.grid_master)[k];
+        float4 e4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (ea > 0.0f) e4 = reinterpret_cast<const float4*>(net.grid_ema)[k];
+        float2 m2[2] = {make_float2(m4.x, m4.y), make_float2(m4.z, m4.w)};
+        float2 v2[2] = {make_float2(v4.x, v4.y), make_float2(v4.z, v4.w)};
+        float2 p2[2] = {make_float2(p4.x, p4.y), make_float2(p4.z, p4.w)};
+        float2 e2[2] = {make_float2(e4.x, e4.y), make_float2(e4.z, e4.w)};
+        bool moved[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const ulonglong2 gi = g2[h];
+            float2 &m = m2[h], &v = v2[h], &p = p2[h], &e = e2[h];
+            moved[h] = !(gi.x == 0ull && gi.y == 0ull && m.x == 0.0f && m.y == 0.0f);
+            if (!moved[h]) continue;
             const float2 gr = make_float2(g_unfix(gi.x), g_unfix(gi.y));
-            float2 m = net.grid_m[j], v = net.grid_v[j], p = net.grid_master[j];
-            m.x = b1 * m.x + (1.0f - b1) * gr.x; m.y = b1 * m.y + (1.0f - b1) * gr.y;
-            v.x = b2 * v.x + (1.0f - b2) * gr.x * gr.x; v.y = b2 * v.y + (1.0f - b2) * gr.y * gr.y;
+            m.x = blend_second(b1, m.x, 1.0f - b1, gr.x); m.y = blend_second(b1, m.y, 1.0f - b1, gr.y);
+            v.x = square_second(b2, v.x, gr.x); v.y = square_second(b2, v.y, gr.y);
             p.x -= lr_g * (m.x / bc1) / (sqrtf(v.x / bc2) + eps);
             p.y -= lr_g * (m.y / bc1) / (sqrtf(v.y / bc2) + eps);
-            net.grid_m[j] = m; net.grid_v[j] = v; net.grid_master[j] = p;
-            reinterpret_cast<ulonglong2*>(net.grid_grad)[j] = make_ulonglong2(0ull, 0ull);
+            if (ea > 0.0f) {
+                e.x = blend_second(ea, e.x, eb, p.x);
+                e.y = blend_second(ea, e.y, eb, p.y);
+            }
+        }
+        if (!moved[0] && !moved[1]) continue;
+        reinterpret_cast<float4*>(net.grid_m)[k] = make_float4(m2[0].x, m2[0].y, m2[1].x, m2[1].y);
+        reinterpret_cast<float4*>(net.grid_v)[k] = make_float4(v2[0].x, v2[0].y, v2[1].x, v2[1].y);
+        reinterpret_cast<float4*>(net.grid_master)[k] = make_float4(p2[0].x, p2[0].y, p2[1].x, p2[1].y);
+        if (ea > 0.0f) reinterpret_cast<float4*>(net.grid_ema)[k] = make_float4(e2[0].x, e2[0].y, e2[1].x, e2[1].y);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!moved[h]) continue;
+            const size_t j = 2 * k + h;
+            if (g2[h].x != 0ull || g2[h].y != 0ull)
+                reinterpret_cast<ulonglong2*>(net.grid_grad)[j] = make_ulonglong2(0ull, 0ull);
             // the FP16 pair table: this entry's own slot and the neighbour slot of the entry before it
-            const __half2 hp = __floats2half2_rn(p.x, p.y);
             const size_t prev = (j & ~static_cast<size_t>(kGTable - 1)) | ((j + kGTable - 1) & (kGTable - 1));
+            const __half2 hp = __floats2half2_rn(p2[h].x, p2[h].y);
             reinterpret_cast<__half2*>(net.grid + j)[0] = hp;
             reinterpret_cast<__half2*>(net.grid + prev)[1] = hp;
             if (ea > 0.0f) {
-                float2 e = net.grid_ema[j];
-                e.x = ea * e.x + eb * p.x;
-                e.y = ea * e.y + eb * p.y;
-                net.grid_ema[j] = e;
-                const __half2 he = __floats2half2_rn(e.x, e.y);
+                const __half2 he = __floats2half2_rn(e2[h].x, e2[h].y);
                 reinterpret_cast<__half2*>(net.grid_inf + j)[0] = he;
                 reinterpret_cast<__half2*>(net.grid_inf + prev)[1] = he;
             }
