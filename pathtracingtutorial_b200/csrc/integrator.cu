@@ -1554,12 +1554,9 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
                                                                          gs->sample_cap, mb, nmb, step_cap, gs->rows);
                         k_guide_dw<<<dim3(kGDwChunks, 4), 128, 0, st>>>(gs->counters, gs->sample_cap, mb, nmb, step_cap,
                                                                         gs->rows, gs->partial);
-                        k_guide_dw_reduce<<<(kGWeights + 255) / 256, 256, 0, st>>>(gs->counters, gs->sample_cap, mb, nmb,
-                                                                                   step_cap, gs->partial,
-                                                                                   gs->net.w_grad);
                         k_guide_adam<<<wf.sms * 8, 256, 0, st>>>(gs->net, gs->counters, gs->sample_cap, mb, nmb,
-                                                                 gs->step, gs->lr, gs->lr, 0.9f, 0.99f, 1e-10f,
-                                                                 gs->lr_half_life, gs->lr_floor);
+                                                                 step_cap, gs->partial, gs->step, gs->lr, gs->lr,
+                                                                 0.9f, 0.99f, 1e-10f, gs->lr_half_life, gs->lr_floor);
                     }
                     k_guide_step<<<1, 1, 0, st>>>(gs->counters, gs->step, gs->net.loss, gs->net.loss_fix,
                                                   gs->sample_cap, nmb);
@@ -2042,7 +2039,7 @@ int integrator_launch(pt_integrator* integ, pt_film* film, pt_scene* s, const pt
     wf.kernel_launches += 1 + passes * (1 + 4 * static_cast<uint64_t>(P.max_depth));
     if (P.gmix)
         wf.kernel_launches += passes * ((wf.guide->infer == PT_GUIDE_INFER_FUSED ? 1 : 3) * P.max_depth +
-                                        (P.grec ? 5 + 4 * guide_minibatches(int64_t(P.npix) * lanes, wf.guide->paths_per_step) : 0));
+                                        (P.grec ? 5 + 3 * guide_minibatches(int64_t(P.npix) * lanes, wf.guide->paths_per_step) : 0));
     return PT_OK;
 }
 
