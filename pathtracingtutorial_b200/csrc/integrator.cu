@@ -806,18 +806,19 @@ __device__ __forceinline__ void push_continuation(const WaveParams& P, int q, bo
 // hands the shading point to the back in the queue entry's own slots:
 // hit[i] = (point, prim | entering << 30, or -1 when the path needs no
 // sampling), ray_o[q][i] = (geometric normal, roulette weight).  Both hold 24
-// warps per SM (80 registers).
+// warps per SM (80 registers), the textured ones 32 (64 registers).
 //
 // They wait for instructions more than for anything else: the code is 66 to
 // 110 KB, and warps at different places in it evict one another's lines.  So
 // the warps of a block start every queue entry together (a barrier a tile),
-// in blocks of 256, and of 768 -- the whole SM in step -- for the textured
+// in blocks of 256, and of 1024 -- the whole SM in step -- for the textured
 // kernels, whose code is the longest.  Shading stage, blocks of 128 without
-// the barrier -> this: Cornell box 512 x 512, 64 spp 10.1 -> 9.7 ms; textured
-// Cornell box 803 x 601, 32 spp 18.4 -> 12.8 ms (256: 14.3, 384: 13.6); closed
-// room 1024 x 1024, 64 spp 73 -> 71 ms (768: 75).
-constexpr int shade_block(bool textured) { return textured ? 768 : 256; }
-constexpr int kShadeThreads = 768;   // per SM
+// the barrier -> this: Cornell box 512 x 512, 64 spp 10.1 -> 9.7 ms (32 warps
+// an SM: 10.2); textured Cornell box 803 x 601, 32 spp 18.4 -> 12.1 ms (768
+// threads an SM in one block: 12.8, in blocks of 256: 14.3); closed room 1024
+// x 1024, 64 spp 73 -> 71 ms (one block: 75; 32 warps: 75.6).
+constexpr int shade_block(bool textured) { return textured ? 1024 : 256; }
+constexpr int shade_threads(bool textured) { return textured ? 1024 : 768; }   // per SM
 constexpr uint32_t kEnteringBit = 0x40000000u;
 
 // Splits a block's share of a queue into hits and misses: tiles are read into
@@ -867,7 +868,7 @@ struct HitMissFeed {
 // full HD, 4 spp.  Without an environment few rays escape, and the split only
 // costs (closed room 71 -> 72.5 ms).
 template <bool Guided, bool Textured, bool Split>
-__global__ void __launch_bounds__(shade_block(Textured), kShadeThreads / shade_block(Textured))
+__global__ void __launch_bounds__(shade_block(Textured), shade_threads(Textured) / shade_block(Textured))
 k_shade_front(WaveParams P, int q, int depth, int s0) {
     const uint32_t cap = static_cast<uint32_t>(P.npath);
     const uint32_t n = min(P.counts[q], cap);
@@ -942,7 +943,7 @@ k_shade_front(WaveParams P, int q, int depth, int s0) {
 }
 
 template <bool Guided, bool Textured>
-__global__ void __launch_bounds__(shade_block(Textured), kShadeThreads / shade_block(Textured))
+__global__ void __launch_bounds__(shade_block(Textured), shade_threads(Textured) / shade_block(Textured))
 k_shade_back(WaveParams P, int q, int depth, int s0) {
     const uint32_t cap = static_cast<uint32_t>(P.npath);
     const uint32_t n = min(P.counts[4], cap);
@@ -1517,7 +1518,7 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
             // the shadow queue is about to be written again
             if (overlap && d > 0) PT_CU(cudaStreamWaitEvent(st, wf.join, 0));
             const bool tex = P.scene.num_textures > 0, guided = P.gmix != nullptr;
-            const int sb = shade_block(tex), sgrid = wf.sms * (kShadeThreads / sb);
+            const int sb = shade_block(tex), sgrid = wf.sms * (shade_threads(tex) / sb);
             auto shadow = [&](cudaStream_t s) {
                 shadow_kernel(walk, tsi)<<<wf.grid_shadow[walk][tsi], trace_block(walk, tsi), 0, s>>>(P, q);
             };
