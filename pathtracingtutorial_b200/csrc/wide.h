@@ -267,8 +267,8 @@ static __device__ __noinline__ uint32_t any_binary(BinaryView b, float ox, float
 // How a warp divides its time.  Its lanes walk different rays, so at any
 // moment some stand on inner nodes, some at a leaf, some are out of work.  A
 // warp keeps stepping through inner nodes while at least kWideInnerMin of its
-// lanes (kWideAnyInnerMin for shadow rays) stand on one, two steps a vote for
-// the longer closest-hit walks; below that the lanes at leaves test their
+// lanes (kWideAnyInnerMin for shadow rays) stand on one, two steps a vote;
+// below that the lanes at leaves test their
 // triangles.  Finished rays are stored, and new ones set up, once kWideFetchMin
 // lanes are out of work.  The walks are bound by issue slots: 16.7 of 32 lanes
 // active, 68 % of slots used (closed 200k-triangle room, second bounce).
@@ -276,7 +276,7 @@ static __device__ __noinline__ uint32_t any_binary(BinaryView b, float ox, float
 // the loop was built up: binary tree, all lanes to a leaf before any tests it
 // 139 / 80 ms; four-wide tree, threshold 16, refill at once 101 / 63 ms; 64
 // registers 94 / 63 ms; contiguous chunks 91 / 59 ms; no order for shadow rays
-// 91 / 47 ms; two steps a vote, threshold 20 90 / 47 ms.  Thresholds 8 to 24
+// 91 / 47 ms; two steps a vote, threshold 20 90 / 46 ms.  Thresholds 8 to 24
 // and refills at 1 to 12 lanes lie within 6 %.
 constexpr int kWideInnerMin = 20, kWideAnyInnerMin = 16, kWideFetchMin = 4;
 
@@ -427,6 +427,24 @@ __device__ __forceinline__ void wide_any_loop(const DeviceScene& s, uint32_t n, 
     int sp = 0;
     uint32_t ref = kNoRef, i = 0;
     bool open = false, hit = false;
+    // one inner node: the last child hit is next, the others go on the stack
+    auto step = [&] {
+        const WideRegs nd = load_wide(s.wide + ref);
+        float t[4];
+        const uint32_t h = wide_boxes(nd, w, tmax, t);
+        ref = kNoRef;
+        if (sp + 3 > Depth) {
+            err |= kErrStackOverflow;
+            return;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (h & (1u << c)) {
+                if (ref != kNoRef) stack[sp++] = ref;
+                ref = nd.ref[c];
+            }
+        if (ref == kNoRef && sp > 0) ref = stack[--sp];
+    };
     for (;;) {
         const uint32_t idle = __ballot_sync(0xffffffffu, ref == kNoRef);
         if (__popc(idle) >= kWideFetchMin) {
@@ -454,23 +472,9 @@ __device__ __forceinline__ void wide_any_loop(const DeviceScene& s, uint32_t n, 
             __syncwarp();
         }
         while (go_on(ref, kWideAnyInnerMin)) {
-            if (!(ref & kLeafBit)) {
-                const WideRegs nd = load_wide(s.wide + ref);
-                float t[4];
-                const uint32_t h = wide_boxes(nd, w, tmax, t);
-                ref = kNoRef;
-                if (sp + 3 > Depth) {
-                    err |= kErrStackOverflow;
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (h & (1u << c)) {
-                            if (ref != kNoRef) stack[sp++] = ref;
-                            ref = nd.ref[c];
-                        }
-                    if (ref == kNoRef && sp > 0) ref = stack[--sp];
-                }
-            }
+            if (!(ref & kLeafBit)) step();
+            __syncwarp();
+            if (!(ref & kLeafBit)) step();
             __syncwarp();
         }
         if ((ref & kLeafBit) && ref != kNoRef) {
