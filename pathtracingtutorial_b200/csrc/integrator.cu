@@ -17,7 +17,7 @@
 //
 // Kernels grid-stride over a queue length that lives in device memory, so a
 // whole batch (sample_per_frame passes x max_depth bounces) is a fixed launch
-// sequence that is captured once into a CUDA graph and replayed.
+// sequence; one that comes again is captured into a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
