@@ -1748,7 +1748,10 @@ int upload_scene(pt_scene* s, int device) {
             PT_CU(cudaMemcpy2DToArray(static_cast<cudaArray_t>(d.tex_arrays[i]), 0, 0, t.rgba.data(), pitch, pitch,
                                       t.height, cudaMemcpyHostToDevice));
         }
-        return build_wide(ts, static_cast<uint32_t>(hs.faces.size()), d);
+        // the same arrays, so the same four-wide tree: it stays as it is, and a
+        // render in flight goes on reading it (whatever changes the arrays frees
+        // the device scene)
+        return PT_OK;
     }
     free_scene_device(s);
     if (int rc = ensure_device(device)) return rc;

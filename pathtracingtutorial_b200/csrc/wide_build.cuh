@@ -254,8 +254,9 @@ __global__ void __launch_bounds__(128) k_wide_tris(const InnerNode* __restrict__
     }
 }
 
-// (Re)builds the wide tree of an uploaded scene from its binary tree on the
-// device.  Scratch lives where the triangle records go afterwards.
+// Builds the wide tree of a scene from its binary tree on the device, once per
+// upload of new arrays: nothing reads d.wide and d.wtris yet.  Scratch lives
+// where the triangle records go afterwards.
 static int build_wide(const SceneTables& t, uint32_t n_faces, DeviceSceneBuffers& d) {
     d.wide_on = false;
     d.wide_need = 0;
