@@ -31,10 +31,12 @@
 // Codes: D(code) is the float with code at bits 16-23 under exponent byte
 // 0x43: 128 + code below 128, 2 * code above, so one byte permute makes the
 // float and the values stay exact.  The two halves of the grid have steps 1
-// and 2.
+// and 2.  Planes are rounded outwards (wide_box.h), so a stored box holds the
+// exact one.
 #pragma once
 
 #include "traverse.h"
+#include "wide_box.h"
 
 namespace ptb {
 

@@ -158,36 +158,6 @@ __global__ void __launch_bounds__(128, 4) k_wide_collapse(const InnerNode* __res
     for (uint32_t i = tid; i < ni; i += stride) sc.index[i] = sc.mark[i] ? 1u : 0u;
 }
 
-__device__ __forceinline__ float wide_decode(uint32_t code) { return __uint_as_float(0x43000000u | (code << 16)); }
-
-// One axis of a node: base and scale that hold [mn, mx].
-__device__ __forceinline__ void wide_frame(float mn, float mx, float& base, uint32_t& exponent) {
-    const float ext = __fsub_ru(mx, mn);
-    int e = ext > 0.0f ? ilogbf(ext / 382.0f) : -100;
-    e = max(-100, min(e, 100));
-    for (int k = 0; k < 4; ++k, ++e) {
-        const float s = __uint_as_float(static_cast<uint32_t>(e + 127) << 23);
-        base = __fsub_rd(mn, 128.0f * s);
-        exponent = static_cast<uint32_t>(e + 127);
-        if (__fmaf_rd(510.0f, s, base) >= mx) break;
-    }
-}
-// Largest code whose plane is at or below v / smallest at or above v.
-__device__ __forceinline__ uint32_t wide_code_lo(float v, float base, float s) {
-    const float x = (v - base) / s;
-    int c = x < 256.0f ? static_cast<int>(floorf(x)) - 128 : static_cast<int>(floorf(0.5f * x));
-    c = max(0, min(c + 1, 255));
-    while (c > 0 && __fmaf_ru(wide_decode(static_cast<uint32_t>(c)), s, base) > v) --c;
-    return static_cast<uint32_t>(c);
-}
-__device__ __forceinline__ uint32_t wide_code_hi(float v, float base, float s) {
-    const float x = (v - base) / s;
-    int c = x <= 255.0f ? static_cast<int>(ceilf(x)) - 128 : static_cast<int>(ceilf(0.5f * x));
-    c = max(0, min(c - 1, 255));
-    while (c < 255 && __fmaf_rd(wide_decode(static_cast<uint32_t>(c)), s, base) < v) ++c;
-    return static_cast<uint32_t>(c);
-}
-
 __global__ void __launch_bounds__(128) k_wide_emit(const InnerNode* __restrict__ inner, uint32_t ni, WideScratch sc,
                                                    WideNode* __restrict__ out) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ni; i += gridDim.x * blockDim.x) {
@@ -210,8 +180,8 @@ __global__ void __launch_bounds__(128) k_wide_emit(const InnerNode* __restrict__
             float mn = b[0].lo[a], mx = b[0].hi[a];
             for (uint32_t c = 1; c < cnt; ++c) { mn = fminf(mn, b[c].lo[a]); mx = fmaxf(mx, b[c].hi[a]); }
             uint32_t e = 0;
-            wide_frame(mn, mx, w.base[a], e);
-            const float s = __uint_as_float(e << 23);
+            if (!wide_frame(mn, mx, w.base[a], e)) sc.status->bad = 1u;
+            const float s = wide_scale(e);
             w.exps |= e << (8 * a);
             w.qlo[a] = w.qhi[a] = 0u;
             for (uint32_t c = 0; c < cnt; ++c) {
@@ -319,8 +289,8 @@ static int build_wide(const SceneTables& t, uint32_t n_faces, DeviceSceneBuffers
                                           nullptr));
         PT_CU(cub::DeviceScan::ExclusiveSum(tmp, scan_tmp, sc.index, sc.index, static_cast<int>(ni)));
         const int wide_grid = static_cast<int>(std::min<uint32_t>((ni + 127) / 128, static_cast<uint32_t>(sms) * 16u));
-        PT_CU(cudaMemcpyAsync(&st, sc.status, sizeof(st), cudaMemcpyDeviceToHost));
         k_wide_emit<<<wide_grid, 128>>>(inner, ni, sc, static_cast<WideNode*>(d.wide));
+        PT_CU(cudaMemcpyAsync(&st, sc.status, sizeof(st), cudaMemcpyDeviceToHost));   // (the records go over it)
     }
     k_wide_tris<<<static_cast<int>(std::min<uint32_t>((2 * ni + 128) / 128, static_cast<uint32_t>(sms) * 16u)), 128>>>(
         inner, ni, root, static_cast<const TriRecord*>(d.tris), n_faces, static_cast<WideTri*>(d.wtris));
