@@ -169,7 +169,8 @@ typedef struct pt_scene_info {
     uint32_t frame_count;
     uint64_t device_bytes;
     uint32_t num_textures;           /* material textures (HostScene::textures) */
-    uint32_t _pad;
+    uint32_t walk_entries;           /* uploaded scenes: stack entries that a walk of the
+                                        four-wide tree may need; 0: rays take the binary tree */
 } pt_scene_info;
 
 typedef struct pt_render_stats {

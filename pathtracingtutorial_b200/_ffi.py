@@ -99,7 +99,7 @@ class SceneInfo(C.Structure):
                 ("num_punctual_lights", C.c_uint32), ("env_width", C.c_int32), ("env_height", C.c_int32),
                 ("bvh_max_depth", C.c_uint32), ("num_inner_nodes", C.c_uint32), ("num_leaves", C.c_uint32),
                 ("frame_count", C.c_uint32), ("device_bytes", C.c_uint64), ("num_textures", C.c_uint32),
-                ("_pad", C.c_uint32)]
+                ("walk_entries", C.c_uint32)]
 
 
 class TuneReport(C.Structure):

@@ -323,6 +323,7 @@ int pt_scene_info_get(const pt_scene* s, pt_scene_info* info) {
     info->frame_count = s->frame_count;
     info->device_bytes = s->dev.bytes;
     info->num_textures = static_cast<uint32_t>(s->host.textures.size());
+    info->walk_entries = s->dev.wide_on ? std::max(s->dev.wide_need, 1u) : 0u;
     return PT_OK;
 }
 
