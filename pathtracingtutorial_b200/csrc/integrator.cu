@@ -817,8 +817,22 @@ __device__ __forceinline__ void push_continuation(const WaveParams& P, int q, bo
 // an SM: 10.2); textured Cornell box 803 x 601, 32 spp 18.4 -> 12.1 ms (768
 // threads an SM in one block: 12.8, in blocks of 256: 14.3); closed room 1024
 // x 1024, 64 spp 73 -> 71 ms (one block: 75; 32 warps: 75.6).
-constexpr int shade_block(bool textured) { return textured ? 1024 : 256; }
-constexpr int shade_threads(bool textured) { return textured ? 1024 : 768; }   // per SM
+//
+// A block of 1024 needs a queue that keeps every SM busy for several tiles: n
+// entries occupy n / 1024 SMs, and the later bounces' queues are a fraction of
+// the first's.  Below six tiles an SM the textured kernels come in blocks of
+// 256.  One frame of the textured Cornell box, depth 8, blocks of 256 / of
+// 1024: 192 x 192 0.51 / 0.66 ms, 512 x 512 0.74 / 0.85 ms, 768 x 512 at 2
+// samples 1.19 / 1.28 ms, 512 x 512 at 4 samples (1.05M paths) 1.96 / 1.93 ms,
+// 1024 x 1024 at 4 samples 6.7 / 6.1 ms; with a guide 512 x 512 at 2 samples
+// 1.85 / 1.92 ms, at 4 samples 3.17 / 3.07 ms.  Both have 64 registers: with
+// 80 the short ones are no faster and the guided front or back kernel fuses
+// other products, so that an image depends on which ran.
+constexpr int kShadeBlock = 256, kShadeBlockLong = 1024, kShadeLongTiles = 6;
+constexpr int shade_blocks(bool textured, int block) { return (textured ? 1024 : 768) / block; }   // per SM
+inline int shade_block(bool textured, int npath, int sms) {
+    return textured && npath >= kShadeLongTiles * kShadeBlockLong * sms ? kShadeBlockLong : kShadeBlock;
+}
 constexpr uint32_t kEnteringBit = 0x40000000u;
 
 // Splits a block's share of a queue into hits and misses: tiles are read into
@@ -867,14 +881,12 @@ struct HitMissFeed {
 // second bounce of the 2M-triangle field: its shading stage 3.4 -> 3.06 ms at
 // full HD, 4 spp.  Without an environment few rays escape, and the split only
 // costs (closed room 71 -> 72.5 ms).
-template <bool Guided, bool Textured, bool Split>
-__global__ void __launch_bounds__(shade_block(Textured), shade_threads(Textured) / shade_block(Textured))
-k_shade_front(WaveParams P, int q, int depth, int s0) {
+template <bool Guided, bool Textured, bool Split, int B>
+__global__ void __launch_bounds__(B, shade_blocks(Textured, B)) k_shade_front(WaveParams P, int q, int depth, int s0) {
     const uint32_t cap = static_cast<uint32_t>(P.npath);
     const uint32_t n = min(P.counts[q], cap);
     const uint32_t sidx0 = P.pass->frame * static_cast<uint32_t>(P.spf) + static_cast<uint32_t>(s0);
     const bool last = depth == P.max_depth - 1;
-    constexpr int B = shade_block(Textured);
     auto shade = [&](const uint32_t i) {
         const uint32_t p = P.queue[q][i];
         if (p >= cap) { atomicOr(P.err, kErrQueueOverflow); return; }
@@ -942,9 +954,8 @@ k_shade_front(WaveParams P, int q, int depth, int s0) {
     }
 }
 
-template <bool Guided, bool Textured>
-__global__ void __launch_bounds__(shade_block(Textured), shade_threads(Textured) / shade_block(Textured))
-k_shade_back(WaveParams P, int q, int depth, int s0) {
+template <bool Guided, bool Textured, int B>
+__global__ void __launch_bounds__(B, shade_blocks(Textured, B)) k_shade_back(WaveParams P, int q, int depth, int s0) {
     const uint32_t cap = static_cast<uint32_t>(P.npath);
     const uint32_t n = min(P.counts[4], cap);
     const uint32_t sidx0 = P.pass->frame * static_cast<uint32_t>(P.spf) + static_cast<uint32_t>(s0);
@@ -1237,17 +1248,21 @@ inline int trace_shape_index(int block, int depth) {
 inline int trace_shape_block(int k) { return k == 6 ? 128 : (k < 2 ? 64 : (k < 4 ? 128 : 256)); }
 
 using ShadeKernel = void (*)(WaveParams, int, int, int);
-inline ShadeKernel shade_front_kernel(bool guided, bool textured, bool split) {
-    if (guided) {
-        if (textured) return split ? k_shade_front<true, true, true> : k_shade_front<true, true, false>;
-        return split ? k_shade_front<true, false, true> : k_shade_front<true, false, false>;
-    }
-    if (textured) return split ? k_shade_front<false, true, true> : k_shade_front<false, true, false>;
-    return split ? k_shade_front<false, false, true> : k_shade_front<false, false, false>;
+template <bool Textured, int B>
+ShadeKernel shade_front_of(bool guided, bool split) {
+    if (guided) return split ? k_shade_front<true, Textured, true, B> : k_shade_front<true, Textured, false, B>;
+    return split ? k_shade_front<false, Textured, true, B> : k_shade_front<false, Textured, false, B>;
 }
-inline ShadeKernel shade_back_kernel(bool guided, bool textured) {
-    if (guided) return textured ? k_shade_back<true, true> : k_shade_back<true, false>;
-    return textured ? k_shade_back<false, true> : k_shade_back<false, false>;
+inline ShadeKernel shade_front_kernel(bool guided, bool textured, bool split, int block) {
+    if (!textured) return shade_front_of<false, kShadeBlock>(guided, split);
+    return block == kShadeBlockLong ? shade_front_of<true, kShadeBlockLong>(guided, split)
+                                    : shade_front_of<true, kShadeBlock>(guided, split);
+}
+inline ShadeKernel shade_back_kernel(bool guided, bool textured, int block) {
+    if (!textured) return guided ? k_shade_back<true, false, kShadeBlock> : k_shade_back<false, false, kShadeBlock>;
+    if (block == kShadeBlockLong)
+        return guided ? k_shade_back<true, true, kShadeBlockLong> : k_shade_back<false, true, kShadeBlockLong>;
+    return guided ? k_shade_back<true, true, kShadeBlock> : k_shade_back<false, true, kShadeBlock>;
 }
 
 using ExtendKernel = void (*)(WaveParams, int, int);
@@ -1518,15 +1533,15 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
             // the shadow queue is about to be written again
             if (overlap && d > 0) PT_CU(cudaStreamWaitEvent(st, wf.join, 0));
             const bool tex = P.scene.num_textures > 0, guided = P.gmix != nullptr;
-            const int sb = shade_block(tex), sgrid = wf.sms * (shade_threads(tex) / sb);
+            const int sb = shade_block(tex, P.npath, wf.sms), sgrid = wf.sms * shade_blocks(tex, sb);
             auto shadow = [&](cudaStream_t s) {
                 shadow_kernel(walk, tsi)<<<wf.grid_shadow[walk][tsi], trace_block(walk, tsi), 0, s>>>(P, q);
             };
             if (int rc = timed(1, [&] {
-                    shade_front_kernel(guided, tex, P.scene.env_tex != 0)<<<sgrid, sb, 0, st>>>(P, q, d, s0);
+                    shade_front_kernel(guided, tex, P.scene.env_tex != 0, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0);
                 })) return rc;
             if (d + 1 < P.max_depth) {
-                if (int rc = timed(1, [&] { shade_back_kernel(guided, tex)<<<sgrid, sb, 0, st>>>(P, q, d, s0); })) return rc;
+                if (int rc = timed(1, [&] { shade_back_kernel(guided, tex, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0); })) return rc;
             }
             if (overlap) {
                 PT_CU(cudaEventRecord(wf.fork, st));
