@@ -1977,10 +1977,20 @@ int integrator_launch(pt_integrator* integ, pt_film* film, pt_scene* s, const pt
     GuideState* gs = wf.guide;
     const pt_render_settings& rs = s->host.settings;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : wf.own_stream;
-    k_begin<<<1, 1, 0, st>>>(P.pass, s->frame_count);
-    PT_CU(cudaGetLastError());
     const bool timing = (rs.flags & PT_FLAG_STAGE_TIMING) != 0;
     const bool use_graph = !timing && !(rs.flags & PT_FLAG_NO_GRAPH);
+    if (use_graph) {
+        // a capture inside a capture is not allowed: refused before anything is
+        // enqueued (PT_FLAG_NO_GRAPH launches can be captured)
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        PT_CU(cudaStreamIsCapturing(st, &capturing));
+        if (capturing != cudaStreamCaptureStatusNone) {
+            set_error("the stream is being captured: render with PT_FLAG_NO_GRAPH");
+            return PT_ERR_CUDA;
+        }
+    }
+    k_begin<<<1, 1, 0, st>>>(P.pass, s->frame_count);
+    PT_CU(cudaGetLastError());
     if (timing) {
         std::vector<StageEvent> ev;
         cudaEvent_t t0, t1;
@@ -2018,14 +2028,6 @@ int integrator_launch(pt_integrator* integ, pt_film* film, pt_scene* s, const pt
         std::memcpy(key.data() + sizeof(WaveParams), &st, sizeof(cudaStream_t));
         std::memcpy(key.data() + sizeof(WaveParams) + sizeof(cudaStream_t), &nframes, sizeof(int));
         std::memcpy(key.data() + sizeof(WaveParams) + sizeof(cudaStream_t) + sizeof(int), &gk, sizeof(GuideKey));
-        // a stream that its owner is capturing stays refused, as a capture inside
-        // a capture is (PT_FLAG_NO_GRAPH launches can be captured)
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        PT_CU(cudaStreamIsCapturing(st, &capturing));
-        if (capturing != cudaStreamCaptureStatusNone) {
-            set_error("the stream is being captured: render with PT_FLAG_NO_GRAPH");
-            return PT_ERR_CUDA;
-        }
         if (key != wf.graph_key) {
             // The first launch of its kind goes out directly; the graph is made
             // when the same launch comes again.  Capturing and instantiating one
