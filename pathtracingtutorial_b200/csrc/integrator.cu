@@ -1980,8 +1980,13 @@ int integrator_launch(pt_integrator* integ, pt_film* film, pt_scene* s, const pt
     const bool timing = (rs.flags & PT_FLAG_STAGE_TIMING) != 0;
     const bool use_graph = !timing && !(rs.flags & PT_FLAG_NO_GRAPH);
     if (use_graph) {
-        // a capture inside a capture is not allowed: refused before anything is
-        // enqueued (PT_FLAG_NO_GRAPH launches can be captured)
+        // The legacy default stream cannot be captured, and a capture inside a
+        // capture is not allowed: refused from the first launch on, before
+        // anything is enqueued (PT_FLAG_NO_GRAPH launches can be captured).
+        if (st == cudaStreamLegacy) {
+            set_error("the legacy default stream cannot be captured: render with PT_FLAG_NO_GRAPH");
+            return PT_ERR_CUDA;
+        }
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         PT_CU(cudaStreamIsCapturing(st, &capturing));
         if (capturing != cudaStreamCaptureStatusNone) {

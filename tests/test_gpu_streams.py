@@ -63,3 +63,12 @@ def test_a_captured_stream_is_refused_and_its_capture_left_alone(launches):
     own.render_batch()
     assert np.array_equal(one, _image(own))
 
+
+def test_the_legacy_stream_is_refused_from_the_first_launch():
+    r = _renderer(1)                                        # cudaStreamLegacy
+    for _ in range(3):
+        with pytest.raises(pt.PTError, match="captur"):
+            r.render_batch()
+    r.scene.update_settings(flags=pt.FLAG_NO_GRAPH)
+    r.render_batch()
+    assert _image(r)[..., :3].max() > 0
