@@ -155,8 +155,10 @@ typedef struct pt_render_settings {
                                    not depend on it. */
     int32_t  trace_block;       /* added: threads per block of the traversal kernels,
                                    64, 128 or 256 (0 = 128) */
-    int32_t  stack_depth;       /* added: traversal stack entries, 32 or 64 (0 = 64); a
-                                   value not above the tree's depth is raised to 64.
+    int32_t  stack_depth;       /* added: traversal stack entries, 32 or 64 (0 = 64);
+                                   raised to 64 or 192 where the walk may need more
+                                   (pt_scene_info.walk_entries; with traversal counters,
+                                   which walk the binary tree, its depth + 1).
                                    pt_autotune sets these three.  Results do not
                                    depend on them. */
 } pt_render_settings;

@@ -18,6 +18,7 @@ void film_free(pt_film* f);
 int  film_clear(pt_film* f);
 int  film_download(const pt_film* f, float* dst, bool fresh, bool host_ptr);
 
+int  walk_entries(const pt_scene* s);   // stack entries of the traversal kernels of a render
 void integrator_free(pt_integrator* integ);
 int  integrator_launch(pt_integrator* integ, pt_film* film, pt_scene* s, const pt_scene_params* prm, int nframes,
                        void* stream);

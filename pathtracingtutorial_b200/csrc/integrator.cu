@@ -401,12 +401,12 @@ enum TraceMode {
     kTraceModes
 };
 
-// Closest hits of queue q.
 // Resident blocks the wide kernels are compiled for: 8 of 128 threads (64
 // registers; left to itself the compiler takes 72 and the closed room's
 // extension stage 101 instead of 97 ms; 56 registers: 97 ms).
 constexpr int wide_blocks(int block, int mode) { return mode == kTraceBinary ? 0 : 1024 / block; }
 
+// Closest hits of queue q.
 template <int Block, int Depth, int Mode>
 __global__ void __launch_bounds__(Block, wide_blocks(Block, Mode)) k_extend(WaveParams P, int q, int depth) {
     const uint32_t n = min(P.counts[q], static_cast<uint32_t>(P.npath));
@@ -1236,16 +1236,22 @@ __global__ void k_bsdf_eval(const pt_material* mats, uint32_t nmat, const float*
     }
 }
 
-// The traversal kernels' shapes: 64, 128 or 256 threads per block with a stack
-// of 32 or 64 entries, and 128 threads with kDeepStack entries for four-wide
-// trees that need more.
+// The traversal kernels' shapes: 64, 128 or 256 threads per block, with a stack
+// of 32 or 64 entries, or of kDeepStack for four-wide trees that need more.
 constexpr int kDeepStack = 192;   // three deferred children a level of the deepest tree accepted
-constexpr int kTraceShapes = 7;
-inline int trace_shape_index(int block, int depth) {
-    if (depth > 64) return 6;
-    return (block == 64 ? 0 : (block == 256 ? 2 : 1)) * 2 + (depth == 32 ? 0 : 1);
+constexpr int kTraceShapes = 9;
+inline int trace_shape(int block, int entries) {
+    return (block == 64 ? 0 : (block == 256 ? 2 : 1)) + (entries == 32 ? 0 : (entries > 64 ? 6 : 3));
 }
-inline int trace_shape_block(int k) { return k == 6 ? 128 : (k < 2 ? 64 : (k < 4 ? 128 : 256)); }
+inline int trace_block(int shape) { return 64 << (shape % 3); }
+
+// How a scene's rays are walked with these settings; traversal counters count
+// the reference's binary walk.
+inline int trace_mode(bool wide_on, int flags) {
+    return !wide_on || (flags & PT_FLAG_COUNT_TRAVERSAL) ? kTraceBinary
+           : (flags & PT_FLAG_WATERTIGHT)                ? kTraceWideWatertight
+                                                         : kTraceWide;
+}
 
 using ShadeKernel = void (*)(WaveParams, int, int, int);
 template <bool Textured, int B>
@@ -1268,41 +1274,35 @@ inline ShadeKernel shade_back_kernel(bool guided, bool textured, int block) {
 using ExtendKernel = void (*)(WaveParams, int, int);
 using ShadowKernel = void (*)(WaveParams, int);
 
-// Kernel of a mode and shape.  The binary walk comes in one shape, the
-// watertight one in the two stack sizes.
-template <int Mode>
-ExtendKernel extend_shape(int k) {
-    switch (k) {
-        case 0: return k_extend<64, 32, Mode>;
-        case 1: return k_extend<64, 64, Mode>;
-        case 2: return k_extend<128, 32, Mode>;
-        case 4: return k_extend<256, 32, Mode>;
-        case 5: return k_extend<256, 64, Mode>;
-        default: return k_extend<128, 64, Mode>;
-    }
+template <int Mode, int Depth>
+ExtendKernel extend_of(int block) {
+    return block == 64 ? k_extend<64, Depth, Mode> : (block == 256 ? k_extend<256, Depth, Mode> : k_extend<128, Depth, Mode>);
 }
-template <int Mode>
-ShadowKernel shadow_shape(int k) {
-    switch (k) {
-        case 0: return k_shadow<64, 32, Mode>;
-        case 1: return k_shadow<64, 64, Mode>;
-        case 2: return k_shadow<128, 32, Mode>;
-        case 4: return k_shadow<256, 32, Mode>;
-        case 5: return k_shadow<256, 64, Mode>;
-        default: return k_shadow<128, 64, Mode>;
-    }
+template <int Mode, int Depth>
+ShadowKernel shadow_of(int block) {
+    return block == 64 ? k_shadow<64, Depth, Mode> : (block == 256 ? k_shadow<256, Depth, Mode> : k_shadow<128, Depth, Mode>);
 }
-inline ExtendKernel extend_kernel(int mode, int k) {
-    if (mode == kTraceBinary) return k_extend<128, 64, kTraceBinary>;
-    if (mode == kTraceWide) return k == 6 ? k_extend<128, kDeepStack, kTraceWide> : extend_shape<kTraceWide>(k);
-    return k == 6 ? k_extend<128, kDeepStack, kTraceWideWatertight> : k_extend<128, 64, kTraceWideWatertight>;
+// (the binary walk never defers more than 64)
+inline ExtendKernel extend_kernel(int mode, int shape) {
+    const int b = trace_block(shape), entries = shape / 3;
+    if (mode == kTraceBinary) return entries == 0 ? extend_of<kTraceBinary, 32>(b) : extend_of<kTraceBinary, 64>(b);
+    if (mode == kTraceWide)
+        return entries == 0 ? extend_of<kTraceWide, 32>(b)
+                            : (entries == 1 ? extend_of<kTraceWide, 64>(b) : extend_of<kTraceWide, kDeepStack>(b));
+    return entries == 0 ? extend_of<kTraceWideWatertight, 32>(b)
+                        : (entries == 1 ? extend_of<kTraceWideWatertight, 64>(b)
+                                        : extend_of<kTraceWideWatertight, kDeepStack>(b));
 }
-inline ShadowKernel shadow_kernel(int mode, int k) {
-    if (mode == kTraceBinary) return k_shadow<128, 64, kTraceBinary>;
-    if (mode == kTraceWide) return k == 6 ? k_shadow<128, kDeepStack, kTraceWide> : shadow_shape<kTraceWide>(k);
-    return k == 6 ? k_shadow<128, kDeepStack, kTraceWideWatertight> : k_shadow<128, 64, kTraceWideWatertight>;
+inline ShadowKernel shadow_kernel(int mode, int shape) {
+    const int b = trace_block(shape), entries = shape / 3;
+    if (mode == kTraceBinary) return entries == 0 ? shadow_of<kTraceBinary, 32>(b) : shadow_of<kTraceBinary, 64>(b);
+    if (mode == kTraceWide)
+        return entries == 0 ? shadow_of<kTraceWide, 32>(b)
+                            : (entries == 1 ? shadow_of<kTraceWide, 64>(b) : shadow_of<kTraceWide, kDeepStack>(b));
+    return entries == 0 ? shadow_of<kTraceWideWatertight, 32>(b)
+                        : (entries == 1 ? shadow_of<kTraceWideWatertight, 64>(b)
+                                        : shadow_of<kTraceWideWatertight, kDeepStack>(b));
 }
-inline int trace_block(int mode, int k) { return mode == kTraceWide ? trace_shape_block(k) : 128; }
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -1323,7 +1323,7 @@ struct Wavefront {
     // launch shapes
     int sms = 0;
     int grid_raygen = 0, grid_finalize = 0;
-    int grid_extend[kTraceModes][kTraceShapes] = {}, grid_shadow[kTraceModes][kTraceShapes] = {};
+    int grid_extend[kTraceModes][kTraceShapes] = {}, grid_shadow[kTraceModes][kTraceShapes] = {};   // trace_shape
     // stats
     unsigned long long host_stats[kStatCount] = {};
     double stage_ms[5] = {0, 0, 0, 0, 0};   // extend, shade, shadow, other, guide
@@ -1402,8 +1402,8 @@ int wavefront_prepare(Wavefront& wf, int device, int npath, int n_slots) {
         wf.grid_raygen = grid_for(reinterpret_cast<const void*>(k_raygen), 256, sms);
         for (int m = 0; m < kTraceModes; ++m)
             for (int k = 0; k < kTraceShapes; ++k) {
-                wf.grid_extend[m][k] = grid_for(reinterpret_cast<const void*>(extend_kernel(m, k)), trace_block(m, k), sms);
-                wf.grid_shadow[m][k] = grid_for(reinterpret_cast<const void*>(shadow_kernel(m, k)), trace_block(m, k), sms);
+                wf.grid_extend[m][k] = grid_for(reinterpret_cast<const void*>(extend_kernel(m, k)), trace_block(k), sms);
+                wf.grid_shadow[m][k] = grid_for(reinterpret_cast<const void*>(shadow_kernel(m, k)), trace_block(k), sms);
             }
         wf.grid_finalize = grid_for(reinterpret_cast<const void*>(k_finalize), 256, sms);
         wf.device = device;
@@ -1505,7 +1505,7 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
     };
     const int lanes = std::max(1, P.npath / std::max(P.npix, 1));
     const int total = static_cast<int>(total_samples);
-    const int tsi = trace_shape_index(P.trace_block, P.stack_depth);
+    const int shape = trace_shape(P.trace_block, P.stack_depth);
     // A bounce's shadow rays only have to be done before the next bounce's NEE
     // writes their queue again, so they run beside its extension rays and guide
     // inference: the long last rays of one launch overlap the other's.  One
@@ -1515,17 +1515,14 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
     // less: the kernels evict one another's code.  Off with stage timing
     // (every launch alone) and in batches, whose items overlap one another.
     const bool overlap = beside && ev == nullptr;
-    // the counters count the reference's binary walk
-    const int walk = !P.scene.wide_on || (P.flags & PT_FLAG_COUNT_TRAVERSAL) ? kTraceBinary
-                     : (P.flags & PT_FLAG_WATERTIGHT)                        ? kTraceWideWatertight
-                                                                             : kTraceWide;
+    const int walk = trace_mode(P.scene.wide_on != 0u, P.flags);
     for (int s0 = 0; s0 < total; s0 += lanes) {
         const int count = std::min(lanes, total - s0);
         if (int rc = timed(3, [&] { k_raygen<<<wf.grid_raygen, 256, 0, st>>>(P, s0, count); })) return rc;
         for (int d = 0; d < P.max_depth; ++d) {
             const int q = d & 1;
             if (int rc = timed(0, [&] {
-                    extend_kernel(walk, tsi)<<<wf.grid_extend[walk][tsi], trace_block(walk, tsi), 0, st>>>(P, q, d);
+                    extend_kernel(walk, shape)<<<wf.grid_extend[walk][shape], trace_block(shape), 0, st>>>(P, q, d);
                 })) return rc;
             if (infer) {
                 if (int rc = timed(4, [&] { launch_guide_infer(*gs, P, q, wf.sms, st); })) return rc;
@@ -1535,7 +1532,7 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
             const bool tex = P.scene.num_textures > 0, guided = P.gmix != nullptr;
             const int sb = shade_block(tex, P.npath, wf.sms), sgrid = wf.sms * shade_blocks(tex, sb);
             auto shadow = [&](cudaStream_t s) {
-                shadow_kernel(walk, tsi)<<<wf.grid_shadow[walk][tsi], trace_block(walk, tsi), 0, s>>>(P, q);
+                shadow_kernel(walk, shape)<<<wf.grid_shadow[walk][shape], trace_block(shape), 0, s>>>(P, q);
             };
             if (int rc = timed(1, [&] {
                     shade_front_kernel(guided, tex, P.scene.env_tex != 0, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0);
@@ -1894,6 +1891,18 @@ void integrator_free(pt_integrator* integ) {
     integ->wf = nullptr;
 }
 
+// Stack entries of the kernels that walk this scene with its settings: what the
+// settings ask for (64 by default), raised to 64 or kDeepStack where the walk may
+// need more -- the binary one as many as the tree is deep, the four-wide one up
+// to three a level.
+int walk_entries(const pt_scene* s) {
+    const pt_render_settings& rs = s->host.settings;
+    const uint32_t want = rs.stack_depth ? static_cast<uint32_t>(rs.stack_depth) : static_cast<uint32_t>(kStackDepth);
+    const uint32_t need = trace_mode(s->dev.wide_on, rs.flags) == kTraceBinary ? s->tables.bvh_depth + 1u : s->dev.wide_need;
+    if (want >= need) return static_cast<int>(want);
+    return need <= static_cast<uint32_t>(kStackDepth) ? kStackDepth : kDeepStack;
+}
+
 // Integrator::launch (Part_2/src/integrators/path.cu:244-255).
 // Sizes the integrator's wavefront for `total` samples per pixel and fills the
 // launch parameters (P, built byte-wise with zeroed padding because its bytes
@@ -1954,14 +1963,9 @@ int prepare_wave(pt_integrator* integ, pt_film* film, pt_scene* s, const pt_scen
         P.galpha = gs->alpha;
         P.grec = gs->mode == PT_GUIDE_TRAIN ? gs->rec : nullptr;
     }
-    // traversal shape: the settings' (the tuner's), 128 threads and 64 entries
-    // by default; a stack no deeper than the tree falls back to 64 entries
+    // traversal shape: the settings' (the tuner's), 128 threads and 64 entries by default
     P.trace_block = rs.trace_block ? rs.trace_block : 128;
-    P.stack_depth = rs.stack_depth ? rs.stack_depth : kStackDepth;
-    if (P.stack_depth <= static_cast<int>(s->tables.bvh_depth)) P.stack_depth = kStackDepth;
-    // (the four-wide walk defers up to three children a level)
-    if (s->dev.wide_on && P.stack_depth < static_cast<int>(s->dev.wide_need))
-        P.stack_depth = s->dev.wide_need <= static_cast<uint32_t>(kStackDepth) ? kStackDepth : kDeepStack;
+    P.stack_depth = walk_entries(s);
     lanes_out = lanes;
     return PT_OK;
 }

@@ -326,16 +326,16 @@ PT_HD bool trace_any(const DeviceScene& s, const RayInv& ray, float tmax, bool w
 // ---------------------------------------------------------------------------
 // Warp-scheduled traversal of the binary tree: renders that count node visits
 // and triangle tests, scenes without a four-wide tree (wide.h), and the
-// allocation-free trace.  Each lane walks its own ray with the visit order, tests and results of trace_closest / trace_any
-// above, but the warp alternates two phases: all lanes that stand on inner
-// nodes step through inner nodes until each reaches a leaf, then all lanes
-// at a leaf test its triangles together.  A lane whose ray is finished takes
-// its next ray (i + stride) at once instead of waiting for the warp's longest
-// ray.  All 32 lanes of the warp must call these loops.
+// allocation-free trace.  Each lane walks its own ray with the visit order,
+// tests and results of trace_closest / trace_any above, but the warp
+// alternates two phases: all lanes that stand on inner nodes step through
+// inner nodes until each reaches a leaf, then all lanes at a leaf test its
+// triangles together.  A lane whose ray is finished takes its next ray
+// (i + stride) at once instead of waiting for the warp's longest ray.  All 32
+// lanes of the warp must call these loops.
 // ---------------------------------------------------------------------------
-// Deferred children of one walk; Depth entries (the tuner picks 32 or 64; a
-// tree needs more entries than its depth only never: the stack holds at most
-// one far child per level).
+// Deferred children of one walk: Depth entries, 32 or 64 (at most one far child
+// a level, so a tree never needs more than its depth).
 template <int Depth = kStackDepth>
 struct StepStack {
     uint32_t ref[Depth];
