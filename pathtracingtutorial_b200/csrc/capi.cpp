@@ -587,7 +587,7 @@ std::string tune_class(const pt_scene* s) {
 
 // One calibration render of `spp` samples per pixel with the scene's current
 // settings, through pt_render's film and integrator: wall milliseconds of the
-// second of two runs (the first captures its graph and sizes its arena).
+// second of two runs (the first sizes its arena).
 int calibration_ms(pt_scene* s, int spp, float* ms) {
     const int w = s->host.camera.width, h = s->host.camera.height;
     std::vector<float> img(static_cast<size_t>(w) * h * 4);
@@ -647,6 +647,9 @@ int pt_autotune(pt_scene* s, int32_t calib_spp, pt_tune_report* report) {
         s->host.settings.paths_in_flight = pif;
         s->host.settings.trace_block = block;
         s->host.settings.stack_depth = depth;
+        // launched directly: the second run of a kind is where a graph would be
+        // captured, about a millisecond that the candidates do not differ in
+        s->host.settings.flags |= PT_FLAG_NO_GRAPH;
         float ms = 0.0f;
         if (int rc = calibration_ms(s, spp, &ms)) { s->host.settings = saved; return rc; }
         const int k = report->candidates++;

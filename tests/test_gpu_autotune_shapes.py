@@ -1,0 +1,31 @@
+"""The tuner's candidates are kernels that differ, timed without a graph capture,
+and its choice is kept per way of walking the rays."""
+import numpy as np
+import pytest
+
+import pathtracingtutorial_b200 as pt
+from pathtracingtutorial_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(n_spheres=60, width=40, height=24, **kw):
+    s = scenes.icosphere_field(n_spheres=n_spheres, subdiv=3, width=width, height=height, spp=4, env_size=(32, 16),
+                               **kw).scene()
+    s.build_accel()
+    s.upload_to_device(0)
+    return s
+
+
+def test_calibration_renders_capture_no_graph():
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    s = _scene(width=41)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        rep = s.autotune(calib_spp=4)
+        torch.cuda.synchronize()
+    names = {e.name for e in prof.events()}
+    assert any("k_extend" in n for n in names) and not rep["cached"]
+    assert not any("cudaGraph" in n for n in names)
+    assert not s.settings().flags & pt.FLAG_NO_GRAPH
