@@ -356,9 +356,10 @@ int pt_render(pt_scene* scene, int32_t spp, float* out_rgba, int32_t out_is_devi
 /* ---- autotuner (no reference counterpart: the reference has fixed launch
  *      shapes).  Times calibration renders of the scene (the pt_render path,
  *      the scene's own settings otherwise) and picks, by coordinate descent,
- *      the traversal stack depth (64, and 32 when the tree is shallower), the
- *      traversal kernels' block size (64, 128, 256) and the wavefront's queue
- *      capacity (paths in flight: 2^24 .. 2^27, as the device holds them).
+ *      the traversal stack depth (64, and 32 where the walk needs no more:
+ *      see pt_render_settings.stack_depth), the traversal kernels' block size
+ *      (64, 128, 256) and the wavefront's queue capacity (paths in flight:
+ *      2^24 .. 2^27, as the device holds them).
  *      The choice is written into the scene's render settings (trace_block,
  *      stack_depth, paths_in_flight), so pt_render and pt_render_batch use it,
  *      and cached per device and scene class (triangles, pixels and depth,

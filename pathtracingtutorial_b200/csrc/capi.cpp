@@ -575,14 +575,23 @@ std::unordered_map<std::string, pt_tune_report>& tune_cache() {
 
 int log2_floor(uint64_t v) { int b = 0; while (v > 1) { v >>= 1; ++b; } return b; }
 
+// Whether a stack of 32 entries stays one (walk_entries).
+bool keeps_to_32(pt_scene* s) {
+    const int asked = s->host.settings.stack_depth;
+    s->host.settings.stack_depth = 32;
+    const bool keeps = walk_entries(s) == 32;
+    s->host.settings.stack_depth = asked;
+    return keeps;
+}
+
 // device : triangles : pixels : depth : sampler : environment : textures : shallow tree
-std::string tune_class(const pt_scene* s) {
+std::string tune_class(pt_scene* s) {
     const HostScene& h = s->host;
     return std::to_string(s->dev.device) + ":" + std::to_string(log2_floor(h.faces.size())) + ":" +
            std::to_string(log2_floor(uint64_t(h.camera.width) * uint64_t(h.camera.height))) + ":" +
            std::to_string(h.settings.max_depth) + ":" + std::to_string(h.settings.sampler_type) + ":" +
            std::to_string(h.env_w > 0 ? 1 : 0) + ":" + std::to_string(h.textures.empty() ? 0 : 1) + ":" +
-           std::to_string(s->tables.bvh_depth < 32 ? 1 : 0);
+           std::to_string(keeps_to_32(s) ? 1 : 0);
 }
 
 // One calibration render of `spp` samples per pixel with the scene's current
@@ -661,10 +670,11 @@ int pt_autotune(pt_scene* s, int32_t calib_spp, pt_tune_report* report) {
         if (ms < best_ms) { best_ms = ms; best = s->host.settings; }
         return PT_OK;
     };
-    // 1) stack depth, 2) block size, 3) queue capacity -- each at the best so far
+    // 1) stack depth (32 only where the walk keeps to it), 2) block size, 3) queue
+    // capacity -- each at the best so far
     const int pif0 = best.paths_in_flight;
     if (int rc = attempt(pif0, 128, 64)) return rc;
-    if (s->tables.bvh_depth < 32)
+    if (keeps_to_32(s))
         if (int rc = attempt(pif0, 128, 32)) return rc;
     const int depth = best.stack_depth;
     for (int block : {64, 256})

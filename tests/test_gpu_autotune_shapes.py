@@ -29,3 +29,16 @@ def test_calibration_renders_capture_no_graph():
     assert any("k_extend" in n for n in names) and not rep["cached"]
     assert not any("cudaGraph" in n for n in names)
     assert not s.settings().flags & pt.FLAG_NO_GRAPH
+
+
+def test_no_candidate_runs_as_another():
+    s = _scene()
+    # a shallow tree whose four-wide walk still needs more than 32 entries
+    assert s.info()["bvh_max_depth"] < 32 < s.info()["walk_entries"] <= 64
+    rep = s.autotune(calib_spp=4)
+    assert not rep["cached"] and {c["stack_depth"] for c in rep["candidates"]} == {64}
+    t = scenes.cornell_box(width=40, height=24, spp=4, max_depth=4).scene()
+    t.build_accel()
+    t.upload_to_device(0)
+    assert t.info()["walk_entries"] <= 32
+    assert {c["stack_depth"] for c in t.autotune(calib_spp=4)["candidates"]} == {32, 64}
