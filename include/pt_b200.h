@@ -363,7 +363,8 @@ int pt_render(pt_scene* scene, int32_t spp, float* out_rgba, int32_t out_is_devi
  *      The choice is written into the scene's render settings (trace_block,
  *      stack_depth, paths_in_flight), so pt_render and pt_render_batch use it,
  *      and cached per device and scene class (triangles, pixels and depth,
- *      each by its power of two; sampler; environment; textures): a later
+ *      each by its power of two; sampler; environment; textures; watertight
+ *      test, traversal counters, the tree that is walked): a later
  *      call for a scene of the same class applies it without timing
  *      (cached = 1).  calib_spp: samples per pixel of a calibration render
  *      (0: enough to fill the largest queue once, at most 256).  Images do not

@@ -584,14 +584,15 @@ bool keeps_to_32(pt_scene* s) {
     return keeps;
 }
 
-// device : triangles : pixels : depth : sampler : environment : textures : shallow tree
-std::string tune_class(pt_scene* s) {
+// device : triangles : pixels : depth : sampler : environment : textures : shallow tree : walk
+std::string tune_class(const pt_scene* s) {
     const HostScene& h = s->host;
     return std::to_string(s->dev.device) + ":" + std::to_string(log2_floor(h.faces.size())) + ":" +
            std::to_string(log2_floor(uint64_t(h.camera.width) * uint64_t(h.camera.height))) + ":" +
            std::to_string(h.settings.max_depth) + ":" + std::to_string(h.settings.sampler_type) + ":" +
            std::to_string(h.env_w > 0 ? 1 : 0) + ":" + std::to_string(h.textures.empty() ? 0 : 1) + ":" +
-           std::to_string(keeps_to_32(s) ? 1 : 0);
+           std::to_string(s->tables.bvh_depth < 32 ? 1 : 0) + ":" + std::to_string(s->dev.wide_on ? 1 : 0) + ":" +
+           std::to_string(h.settings.flags & (PT_FLAG_WATERTIGHT | PT_FLAG_COUNT_TRAVERSAL));
 }
 
 // One calibration render of `spp` samples per pixel with the scene's current

@@ -32,7 +32,7 @@ def test_calibration_renders_capture_no_graph():
 
 
 def test_no_candidate_runs_as_another():
-    s = _scene()
+    s = _scene(height=48)
     # a shallow tree whose four-wide walk still needs more than 32 entries
     assert s.info()["bvh_max_depth"] < 32 < s.info()["walk_entries"] <= 64
     rep = s.autotune(calib_spp=4)
@@ -42,3 +42,14 @@ def test_no_candidate_runs_as_another():
     t.upload_to_device(0)
     assert t.info()["walk_entries"] <= 32
     assert {c["stack_depth"] for c in t.autotune(calib_spp=4)["candidates"]} == {32, 64}
+
+
+def test_the_choice_is_kept_per_walk():
+    for flags in (0, pt.FLAG_WATERTIGHT, pt.FLAG_COUNT_TRAVERSAL):
+        for cached in (False, True):
+            s = _scene(width=320, height=24, seed=3 + cached)
+            s.update_settings(flags=flags)
+            ref = pt.render(s, 4)
+            assert s.autotune(calib_spp=4)["cached"] == cached
+            assert s.settings().flags == flags
+            assert np.array_equal(pt.render(s, 4), ref)
