@@ -84,6 +84,22 @@ def workload(small: bool):
     return scenes.icosphere_field()
 
 
+def upload_bytes(info):
+    """Bytes that pt_scene_upload copies from the host for a scene without
+    material textures: the binary tree's nodes and triangle records, the mesh,
+    materials, lights, the light tables, the environment and its tables (the
+    four-wide tree is built on the device from these)."""
+    from pathtracingtutorial_b200 import _ffi
+    texels = info["env_width"] * info["env_height"]
+    return int(64 * info["num_inner_nodes"] + 48 * info["num_faces"]
+               + _ffi.VERTEX_DTYPE.itemsize * info["num_vertices"] + _ffi.FACE_DTYPE.itemsize * info["num_faces"]
+               + _ffi.MATERIAL_DTYPE.itemsize * info["num_materials"]
+               + (_ffi.EMISSIVE_DTYPE.itemsize + _ffi.ALIAS_DTYPE.itemsize) * info["num_emissive_triangles"]
+               + 4 * info["num_faces"]                                        # selection probability per triangle
+               + _ffi.PUNCTUAL_DTYPE.itemsize * info["num_punctual_lights"]
+               + (16 + 4 + _ffi.ALIAS_DTYPE.itemsize) * texels)
+
+
 def config_of(sa, spp):
     return {"workload": f"icosphere_field {sa.meta['triangles']} tri, {int(sa.camera['width'])}x"
                         f"{int(sa.camera['height'])}, {spp} spp, depth {sa.max_depth}, sobol, env 2048x1024",
@@ -625,7 +641,7 @@ def ours(args):
         "ray_classes": {"camera": st["camera_rays"] // args.steps, "extension": st["extension_rays"] // args.steps,
                         "shadow": st["shadow_rays"] // args.steps},
         "e2e": {"value": round(e2e_val, 2), "unit": METRIC, "ms_per_step": round(statistics.median(e2e_ms), 2),
-                "h2d_bytes_per_step": int(info["device_bytes"]), "d2h_bytes_per_step": int(img.nbytes),
+                "h2d_bytes_per_step": upload_bytes(info), "d2h_bytes_per_step": int(img.nbytes),
                 "path": "pt_scene_upload + pt_render (host arrays -> device, 256 spp, image -> host)"},
         "roofline": {"kernel": "k_extend (closest-hit traversal)", "bound": "hbm", "achieved": round(achieved, 1),
                      "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
