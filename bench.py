@@ -105,7 +105,7 @@ def config_of(sa, spp):
                         f"{int(sa.camera['height'])}, {spp} spp, depth {sa.max_depth}, sobol, env 2048x1024",
             "triangles": sa.meta["triangles"], "width": int(sa.camera["width"]), "height": int(sa.camera["height"]),
             "spp": spp, "max_depth": sa.max_depth, "sampler": "sobol", "sample_per_frame": sa.sample_per_frame,
-            "l2": "inputs larger than L2 (BVH + triangles ~150 MB > 126 MB L2)"}
+            "l2": "inputs larger than L2 (four-wide tree + triangle records ~170 MB > 126 MB L2)"}
 
 
 def measured_peaks():
@@ -601,17 +601,19 @@ def ours(args):
     per_launch_ms = ist["extend_ms"] / launches
     achieved = alg_bytes / launches / (per_launch_ms / 1e3) / 1e9
     peak, peak_kind = measured_peaks()
-    traffic = units = None
+    traffic = traffic_case = units = None
     tp = os.path.join(ROOT, "profiles", "extend_traffic.json")
     if os.path.exists(tp):
         with open(tp) as f:
             prof = json.load(f)
         traffic = prof.get("dram_bytes_per_launch")
+        traffic_case = {"workload": prof.get("workload"), "launches": prof.get("launches"),
+                        "algorithmic_bytes_per_launch": prof.get("algorithmic_bytes_per_launch")}
         u = prof.get("units_small_case")
         if u:   # the L2 / L1 / issue fractions beside the HBM one (ncu, small case)
             units = {k: u[k] for k in ("l2_throughput_of_peak", "l1tex_throughput_of_peak", "dram_throughput_of_peak",
                                        "issue_active_of_peak", "lanes_per_warp_instruction")}
-            units["source"] = "profiles/extend_traffic.json (ncu --set full, 4-spp case)"
+            units["source"] = "profiles/extend_traffic.json (ncu, metrics by name, 4-spp case)"
     stage_total = ist["extend_ms"] + ist["shade_ms"] + ist["shadow_ms"] + ist["other_ms"]
 
     if rank != 0:
@@ -634,7 +636,7 @@ def ours(args):
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": dict(config_of(sa, spp), launch={
             "paths_in_flight": scene.settings().paths_in_flight, "trace_block": scene.settings().trace_block,
-            "stack_depth": scene.settings().stack_depth,
+            "stack_depth": scene.settings().stack_depth, "walk_entries": info["walk_entries"],
             "autotune": None if tuned is None else {k: tuned[k] for k in ("calib_spp", "best_ms", "default_ms",
                                                                          "candidates")}}),
         "rays_per_step": total_rays / args.steps / world,
@@ -643,16 +645,19 @@ def ours(args):
         "e2e": {"value": round(e2e_val, 2), "unit": METRIC, "ms_per_step": round(statistics.median(e2e_ms), 2),
                 "h2d_bytes_per_step": upload_bytes(info), "d2h_bytes_per_step": int(img.nbytes),
                 "path": "pt_scene_upload + pt_render (host arrays -> device, 256 spp, image -> host)"},
-        "roofline": {"kernel": "k_extend (closest-hit traversal)", "bound": "hbm", "achieved": round(achieved, 1),
+        "roofline": {"kernel": "k_extend (closest-hit traversal)", "bound": "issue", "achieved": round(achieved, 1),
                      "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
-                     "traffic": traffic, "units": units, "algorithmic_bytes_per_launch": alg_bytes / launches,
+                     "traffic": traffic, "traffic_case": traffic_case, "units": units,
+                     "algorithmic_bytes_per_launch": alg_bytes / launches,
                      "avg_launch_ms": round(per_launch_ms, 4), "launches": launches,
                      "stage_ms": {"extend": round(ist["extend_ms"], 2), "shade": round(ist["shade_ms"], 2),
                                   "shadow": round(ist["shadow_ms"], 2), "other": round(ist["other_ms"], 2)},
                      "extend_share": round(ist["extend_ms"] / max(stage_total, 1e-9), 3),
                      "note": "achieved = (32 B x node pops + 36 B x triangle tests of the reference's "
                              "traversal of the same rays) / extend launch time, CUDA events on a stage-timed "
-                             "replica of one step; traffic = ncu dram read+write per launch (profiles/)"},
+                             "replica of one step, over the measured HBM copy rate: a rate of work (the four-wide "
+                             "walk reaches the same hits over fewer bytes, mostly from the caches, and is bound "
+                             "by issue slots: units); traffic = ncu dram read + write per launch of traffic_case"},
         "cpu_baseline": cpu,
         "clocks": clocks.summary(),
         "gpu_launches": int(st["kernel_launches"]),
