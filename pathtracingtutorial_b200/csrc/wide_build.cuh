@@ -251,21 +251,15 @@ static int build_wide(const SceneTables& t, uint32_t n_faces, DeviceSceneBuffers
     // a node with fewer than four children has only leaves below it, so there
     // are at most 2/3 as many wide nodes as binary ones (and one)
     const size_t want_nodes = (size_t(ni) * 2 / 3 + 2) * sizeof(WideNode);
-    auto grow = [&](void*& p, size_t& have, size_t want) -> int {
-        if (p && have >= want) return PT_OK;
-        if (p) cudaFree(p);
-        p = nullptr;
-        have = 0;
-        if (cudaMalloc(&p, want) != cudaSuccess) {
-            cudaGetLastError();
-            p = nullptr;
-            return PT_ERR_NOMEM;
-        }
-        have = want;
+    // without room for both the scene keeps the binary walk
+    if (cudaMalloc(&d.wide, want_nodes) != cudaSuccess || cudaMalloc(&d.wtris, want_tris) != cudaSuccess) {
+        cudaGetLastError();
+        if (d.wide) cudaFree(d.wide);
+        d.wide = d.wtris = nullptr;
         return PT_OK;
-    };
-    // without room for it the scene keeps the binary walk
-    if (grow(d.wide, d.wide_bytes, want_nodes) || grow(d.wtris, d.wtris_bytes, want_tris)) return PT_OK;
+    }
+    d.wide_bytes = want_nodes;
+    d.wtris_bytes = want_tris;
     const InnerNode* inner = static_cast<const InnerNode*>(d.inner);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device);
