@@ -23,10 +23,15 @@
 // and the sum, and of the exact test's own two operations, move the
 // comparison by at most u |inv| (6 |o| + 6.4 M); the near distances are
 // lowered and the far ones raised by 8 u |inv| (|o| + M) (16 u in watertight
-// mode, whose exact exit is scaled by 1 + 8 u).  An axis with a zero or
-// denormal direction component (inv infinite) uses inv = +-2^100, which keeps
-// "inside the slab, its planes included" and rejects outside; rays beyond the
-// ranges this argument needs take the binary walk (wide_ray).
+// mode, whose exact exit is scaled by 1 + 8 u).  An axis with a zero direction
+// component (inv infinite) uses a power of two that puts its pad far above
+// every distance on the other axes, which keeps "inside the slab, its planes
+// included" and rejects outside.  Long directions need no bound of their own: a
+// product below the normal numbers is off by less than 2^-140, and pads are at
+// least 2^-111.  Rays beyond what this argument needs -- denormal components,
+// distances beyond about 2^117, no direction at all -- take the binary walk
+// (wide_ray), out of line and lane by lane: 2M rays of length 1e8 over 512k
+// triangles took 3.6 ms there and take 1.2 here.
 //
 // Codes: D(code) is the float with code at bits 16-23 under exponent byte
 // 0x43: 128 + code below 128, 2 * code above, so one byte permute makes the
@@ -64,9 +69,12 @@ struct alignas(32) WideTri {
 };
 static_assert(sizeof(WideTri) == 64, "WideTri must be 64 bytes");
 
-#if defined(__CUDACC__)
-
-constexpr float kWideInvMin = 9.5367432e-7f, kWideInvMax = 7.5557864e22f, kWideInvInf = 1.2676506e30f;   // 2^-20, 2^76, 2^100
+constexpr float kWideInvMax = 7.5557864e22f;   // 2^76
+constexpr float kWidePadMin = 3.8518599e-34f, kWidePadMax = 1e29f;   // 2^-111; products far from overflow
+// (distances on an axis go up to 2^21 pads; of a flat axis's pad the roundings
+// leave a fifth)
+constexpr float kWideFlatAbove = 16777216.0f;
+constexpr uint32_t kWideLiteral = 8u;           // in WideRay::sgn: an inverse is infinite
 
 // A ray as the wide walk holds it.
 struct WideRay {
@@ -74,70 +82,68 @@ struct WideRay {
     float    ix, iy, iz;        // 1 / d, infinite ones replaced
     float    nx, ny, nz;        // -(o * inv + pad): near planes
     float    fx, fy, fz;        // -(o * inv - pad): far planes
-    uint32_t sgn;               // direction sign bits x | y << 1 | z << 2
+    uint32_t sgn;               // direction sign bits x | y << 1 | z << 2; kWideLiteral
 };
 
-// False when the ray needs the binary walk.
-__device__ __forceinline__ bool wide_ray(const DeviceScene& s, const RayInv& r, bool watertight, WideRay& w) {
+// False when the ray needs the binary walk.  NaN and infinite origins and
+// directions fail by their pads.
+PT_HD bool wide_ray(const DeviceScene& s, const RayInv& r, bool watertight, WideRay& w) {
     w.ox = r.ox; w.oy = r.oy; w.oz = r.oz;
     w.dx = r.dx; w.dy = r.dy; w.dz = r.dz;
     w.ix = r.ix; w.iy = r.iy; w.iz = r.iz;
     w.sgn = static_cast<uint32_t>(r.sx | (r.sy << 1) | (r.sz << 2));
-    // finite inverses from 2^-20 (so that S and the pads stay normal numbers)
-    // to 2^76; an infinite one becomes 2^100 and then dominates every other
-    // distance.  NaN fails.
-    const float lo = fminf(fminf(fabsf(r.ix), fabsf(r.iy)), fabsf(r.iz));
-    const float hi = fmaxf(fmaxf(fabsf(r.ix), fabsf(r.iy)), fabsf(r.iz));
-    bool ok = s.wide_on && lo >= kWideInvMin;
-    if (!(hi <= kWideInvMax)) {
-        auto fix = [&](float& v) {
-            if (fabsf(v) > FLT_MAX) v = copysignf(kWideInvInf, v);
-            else ok = ok && fabsf(v) <= kWideInvMax;   // false for NaN
-        };
-        fix(w.ix); fix(w.iy); fix(w.iz);
-    }
     const float k = watertight ? 9.5367432e-7f : 4.7683716e-7f;   // 16 u, 8 u
+    bool ok = s.wide_on != 0u;
+    if (!(fmaxf(fmaxf(fabsf(r.ix), fabsf(r.iy)), fabsf(r.iz)) <= kWideInvMax)) {
+        // an infinite inverse becomes the power of two that puts the pad at 2^79
+        // to 2^80 (2^126 at most); the pad must then dominate the other axes
+        float flat = FLT_MAX, rest = 0.0f;
+        auto fix = [&](float& v, float d, float o, float most) {
+            const float a = fmaf(fabsf(o), k, most * k);
+            if (d == 0.0f) {
+                const uint32_t e = 333u - (__float_as_uint_hd(a) >> 23);
+                v = copysignf(__uint_as_float_hd((e < 253u ? e : 253u) << 23), v);
+                flat = fminf(flat, a * fabsf(v));
+                w.sgn |= kWideLiteral;
+            } else {
+                ok = ok && fabsf(v) <= kWideInvMax;   // false for NaN and for denormal components
+                rest = fmaxf(rest, a * fabsf(v));
+            }
+        };
+        fix(w.ix, r.dx, r.ox, s.coord_max[0]);
+        fix(w.iy, r.dy, r.oy, s.coord_max[1]);
+        fix(w.iz, r.dz, r.oz, s.coord_max[2]);
+        ok = ok && rest > 0.0f && flat >= kWideFlatAbove * rest;
+    }
     const float px = fmaf(fabsf(r.ox), k, s.coord_max[0] * k) * fabsf(w.ix);
     const float py = fmaf(fabsf(r.oy), k, s.coord_max[1] * k) * fabsf(w.iy);
     const float pz = fmaf(fabsf(r.oz), k, s.coord_max[2] * k) * fabsf(w.iz);
     w.nx = fmaf(-r.ox, w.ix, -px); w.ny = fmaf(-r.oy, w.iy, -py); w.nz = fmaf(-r.oz, w.iz, -pz);
     w.fx = fmaf(-r.ox, w.ix, px); w.fy = fmaf(-r.oy, w.iy, py); w.fz = fmaf(-r.oz, w.iz, pz);
-    // products far from overflow (NaN origins fail)
-    return ok && px < 1e29f && py < 1e29f && pz < 1e29f;
+    return ok && fminf(fminf(px, py), pz) >= kWidePadMin && px < kWidePadMax && py < kWidePadMax && pz < kWidePadMax;
 }
 
-constexpr uint32_t kNoRef = 0xffffffffu;   // a lane without a ray; an unused slot
-
-// One node in registers.  (Volatile: a load that is free to move could move
-// above the test that the lane has a node.)
+// One node in registers.
 struct WideRegs {
     float    bx, by, bz;
     uint32_t exps, lo[3], hi[3], o0, o1, ref[4];
 };
 
-__device__ __forceinline__ WideRegs load_wide(const WideNode* p) {
-    WideRegs n;
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(n.bx), "=f"(n.by), "=f"(n.bz), "=r"(n.exps), "=r"(n.lo[0]), "=r"(n.lo[1]), "=r"(n.lo[2]), "=r"(n.hi[0])
-        : "l"(p));
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(n.hi[1]), "=r"(n.hi[2]), "=r"(n.o0), "=r"(n.o1), "=r"(n.ref[0]), "=r"(n.ref[1]), "=r"(n.ref[2]),
-          "=r"(n.ref[3])
-        : "l"(reinterpret_cast<const char*>(p) + 32));
-    return n;
-}
-
 // D(code of slot c).
 template <int C>
-__device__ __forceinline__ float wide_code(uint32_t q) {
+PT_HD float wide_code(uint32_t q) {
+#if defined(__CUDA_ARCH__)
     return __uint_as_float(__byte_perm(q, 0x43000000u, 0x7044u | (C << 8)));
+#else
+    return wide_decode((q >> (8 * C)) & 255u);
+#endif
 }
 
 // Conservative entry distances of the four slots; returns the slots hit.
-__device__ __forceinline__ uint32_t wide_boxes(const WideRegs& n, const WideRay& r, float best, float (&t)[4]) {
-    const float sx = __uint_as_float((n.exps & 0xffu) << 23) * r.ix;
-    const float sy = __uint_as_float((n.exps & 0xff00u) << 15) * r.iy;
-    const float sz = __uint_as_float((n.exps & 0xff0000u) << 7) * r.iz;
+PT_HD uint32_t wide_boxes(const WideRegs& n, const WideRay& r, float best, float (&t)[4]) {
+    const float sx = __uint_as_float_hd((n.exps & 0xffu) << 23) * r.ix;
+    const float sy = __uint_as_float_hd((n.exps & 0xff00u) << 15) * r.iy;
+    const float sz = __uint_as_float_hd((n.exps & 0xff0000u) << 7) * r.iz;
     const float nx = fmaf(n.bx, r.ix, r.nx), ny = fmaf(n.by, r.iy, r.ny), nz = fmaf(n.bz, r.iz, r.nz);
     const float fx = fmaf(n.bx, r.ix, r.fx), fy = fmaf(n.by, r.iy, r.fy), fz = fmaf(n.bz, r.iz, r.fz);
     const uint32_t qnx = (r.sgn & 1u) ? n.hi[0] : n.lo[0], qfx = (r.sgn & 1u) ? n.lo[0] : n.hi[0];
@@ -156,6 +162,24 @@ __device__ __forceinline__ uint32_t wide_boxes(const WideRegs& n, const WideRay&
     PT_SLOT(0) PT_SLOT(1) PT_SLOT(2) PT_SLOT(3)
 #undef PT_SLOT
     return h & (n.exps >> 24);
+}
+
+#if defined(__CUDACC__)
+
+constexpr uint32_t kNoRef = 0xffffffffu;   // a lane without a ray; an unused slot
+
+// (Volatile: a load that is free to move could move above the test that the
+// lane has a node.)
+__device__ __forceinline__ WideRegs load_wide(const WideNode* p) {
+    WideRegs n;
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(n.bx), "=f"(n.by), "=f"(n.bz), "=r"(n.exps), "=r"(n.lo[0]), "=r"(n.lo[1]), "=r"(n.lo[2]), "=r"(n.hi[0])
+        : "l"(p));
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(n.hi[1]), "=r"(n.hi[2]), "=r"(n.o0), "=r"(n.o1), "=r"(n.ref[0]), "=r"(n.ref[1]), "=r"(n.ref[2]),
+          "=r"(n.ref[3])
+        : "l"(reinterpret_cast<const char*>(p) + 32));
+    return n;
 }
 
 // Slots visited after each slot (nibbles) in this ray's octant.
@@ -186,7 +210,7 @@ template <bool Watertight>
 __device__ __forceinline__ bool wide_leaf_passes(const WideTri* p, const WideRay& w, float best) {
     const float2* b = reinterpret_cast<const float2*>(reinterpret_cast<const char*>(p) + 40);
     const float2 b0 = __ldg(b), b1 = __ldg(b + 1), b2 = __ldg(b + 2);
-    if (fmaxf(fmaxf(fabsf(w.ix), fabsf(w.iy)), fabsf(w.iz)) > kWideInvMax)
+    if (w.sgn & kWideLiteral)
         return wide_leaf_literal(w.ox, w.oy, w.oz, w.dx, w.dy, w.dz, b0, b1, b2, best, exit_scale(Watertight));
     RayInv r;
     r.ox = w.ox; r.oy = w.oy; r.oz = w.oz;

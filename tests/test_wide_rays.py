@@ -1,0 +1,143 @@
+"""The conservative box test of the four-wide walk (csrc/wide.h), compiled for
+the host: for every ray it takes, a child whose exact box passes the reference's
+test is hit and its entry distance is not raised -- over scales, flat axes, zero
+and denormal direction components, short and long directions, both modes."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PROGRAM = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <cmath>
+#include <random>
+#include <algorithm>
+#include "wide.h"
+using namespace ptb;
+
+// argv: scale of the coordinates, scale of the directions, 1: one axis nearly flat, watertight, rays
+int main(int argc, char** argv) {
+    const double cs = atof(argv[1]), ds = atof(argv[2]);
+    const bool flat = atoi(argv[3]) != 0, wt = atoi(argv[4]) != 0;
+    const long n = atol(argv[5]);
+    std::mt19937_64 g(12345);
+    std::uniform_real_distribution<double> u(-1.0, 1.0);
+    std::uniform_int_distribution<int> die(0, 1 << 20);
+    long taken = 0, passed = 0, wrong = 0, hit = 0, slots = 0;
+    for (long k = 0; k < n; ++k) {
+        // four boxes in a cube, often small against it, sometimes without thickness
+        double ax[3] = {cs, cs, cs};
+        if (flat) ax[die(g) % 3] = cs * std::pow(10.0, -30.0 * std::fabs(u(g)));
+        DeviceScene s{};
+        s.wide_on = 1u;
+        float lo[3][4], hi[3][4];
+        WideRegs nd{};
+        nd.exps = 15u << 24;
+        float* base[3] = {&nd.bx, &nd.by, &nd.bz};
+        const double at = std::pow(10.0, -4.0 * std::fabs(u(g))), size = std::pow(10.0, -4.0 * std::fabs(u(g)));
+        for (int a = 0; a < 3; ++a) {
+            s.coord_max[a] = std::max(static_cast<float>(ax[a]), 8.2718061e-25f);
+            const double c0 = u(g) * at;
+            float mn = FLT_MAX, mx = -FLT_MAX;
+            for (int c = 0; c < 4; ++c) {
+                const double c1 = std::min(1.0, std::max(-1.0, c0 + u(g) * size)),
+                             c2 = die(g) % 4 ? std::min(1.0, std::max(-1.0, c1 + u(g) * size)) : c1;
+                lo[a][c] = static_cast<float>(std::min(c1, c2) * ax[a]);
+                hi[a][c] = static_cast<float>(std::max(c1, c2) * ax[a]);
+                lo[a][c] = std::max(lo[a][c], -s.coord_max[a]);
+                hi[a][c] = std::min(hi[a][c], s.coord_max[a]);
+                mn = std::min(mn, lo[a][c]);
+                mx = std::max(mx, hi[a][c]);
+            }
+            uint32_t e = 0;
+            if (!wide_frame(mn, mx, *base[a], e)) return 3;
+            nd.exps |= e << (8 * a);
+            for (int c = 0; c < 4; ++c) {
+                nd.lo[a] |= wide_code_lo(lo[a][c], *base[a], wide_scale(e)) << (8 * c);
+                nd.hi[a] |= wide_code_hi(hi[a][c], *base[a], wide_scale(e)) << (8 * c);
+            }
+        }
+        for (int rep = 0; rep < 4; ++rep) {
+            // towards a point of a box, or anywhere; from inside, outside, far off, a box plane
+            float o[3], d[3];
+            const int c = die(g) & 3, from = die(g) % 8;
+            const double off = std::pow(10.0, 3.0 * u(g));
+            for (int a = 0; a < 3; ++a) {
+                const double f = 0.5 + 0.5 * u(g);
+                const double q = lo[a][c] + f * (static_cast<double>(hi[a][c]) - lo[a][c]);
+                o[a] = static_cast<float>(from == 0 ? lo[a][c] : from == 1 ? hi[a][c] : from == 2 ? q : u(g) * off * ax[a]);
+                d[a] = static_cast<float>((die(g) % 8 ? q - o[a] : u(g) * ax[a]) / cs * ds);
+                if (die(g) % 8 == 0) d[a] = die(g) & 1 ? -0.0f : 0.0f;
+                if (die(g) % 64 == 0) d[a] = 1e-41f;
+                if (die(g) % 8 == 0) o[a] = die(g) & 1 ? lo[a][c] : hi[a][c];
+            }
+            RayInv r = make_ray_inv(o[0], o[1], o[2], d[0], d[1], d[2]);
+            r.xs = exit_scale(wt);
+            WideRay w;
+            if (!wide_ray(s, r, wt, w)) continue;
+            ++taken;
+            float en[4], ex[4];
+            for (int i = 0; i < 4; ++i)
+                box_span(r, lo[0][i], lo[1][i], lo[2][i], hi[0][i], hi[1][i], hi[2][i], en[i], ex[i]);
+            // best: none yet, exactly an entry, a little below one, anything
+            const float b[4] = {FLT_MAX, en[c], nextafterf(en[c], 0.0f),
+                                static_cast<float>(std::fabs(u(g)) * 2.0 * cs / std::max(ds, 1e-30))};
+            for (float best : b) {
+                float t[4];
+                const uint32_t h = wide_boxes(nd, w, best, t);
+                for (int i = 0; i < 4; ++i) {
+                    ++slots;
+                    hit += (h >> i) & 1u;
+                    if (!(en[i] <= best && en[i] <= ex[i])) continue;
+                    ++passed;
+                    if (!((h >> i) & 1u) || !(t[i] <= en[i])) {
+                        if (!wrong++)
+                            std::fprintf(stderr, "box %d t %g entry %g exit %g best %g o %g %g %g d %g %g %g\n", i, t[i],
+                                         en[i], ex[i], best, o[0], o[1], o[2], d[0], d[1], d[2]);
+                    }
+                }
+            }
+        }
+    }
+    std::printf("%ld %ld %ld %ld %ld\n", taken, passed, wrong, hit, slots);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def walk(tmp_path_factory):
+    d = tmp_path_factory.mktemp("wide_rays")
+    (d / "rays.cpp").write_text(PROGRAM)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-mfma", str(d / "rays.cpp"),
+                    "-I", os.path.join(ROOT, "pathtracingtutorial_b200", "csrc"),
+                    "-I", "/usr/local/cuda/include", "-o", str(d / "rays")], check=True)
+
+    def run(*args):
+        r = subprocess.run([str(d / "rays"), *(str(a) for a in args)], capture_output=True, text=True, check=True)
+        return [int(x) for x in r.stdout.split()], r.stderr
+    return run
+
+
+RAYS = 20_000
+
+
+@pytest.mark.parametrize("watertight", [0, 1])
+@pytest.mark.parametrize("flat", [0, 1])
+@pytest.mark.parametrize("dirs", [1e-12, 1.0, 1e8, 1e25])
+@pytest.mark.parametrize("coords", [1e-12, 1e-3, 1.0, 5e6, 1e12, 1e25])
+def test_no_passing_box_is_missed(walk, coords, dirs, flat, watertight):
+    (taken, passed, wrong, hit, slots), first = walk(coords, dirs, flat, watertight, RAYS)
+    assert wrong == 0, first
+    assert taken == 0 or passed > taken // 4        # the rays that are taken do meet boxes
+
+
+@pytest.mark.parametrize("coords,dirs", [(1.0, 1.0), (1.0, 1e8), (5e6, 1.0), (5e6, 1e-3), (1e-3, 1.0), (1.0, 1e25)])
+def test_ordinary_rays_are_taken(walk, coords, dirs):
+    """Axis-parallel rays at large coordinates and long directions among them; one ray in 21 has a denormal
+    component and is not."""
+    (taken, passed, wrong, hit, slots), _ = walk(coords, dirs, 0, 0, RAYS)
+    assert taken > 0.9 * 4 * RAYS
+    assert hit < 2 * passed                          # and the test still rejects
