@@ -1536,10 +1536,8 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
             };
             if (int rc = timed(1, [&] {
                     shade_front_kernel(guided, tex, P.scene.env_tex != 0, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0);
+                    if (d + 1 < P.max_depth) shade_back_kernel(guided, tex, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0);
                 })) return rc;
-            if (d + 1 < P.max_depth) {
-                if (int rc = timed(1, [&] { shade_back_kernel(guided, tex, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0); })) return rc;
-            }
             if (overlap) {
                 PT_CU(cudaEventRecord(wf.fork, st));
                 PT_CU(cudaStreamWaitEvent(wf.side, wf.fork, 0));
