@@ -1538,7 +1538,8 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
                     shade_front_kernel(guided, tex, P.scene.env_tex != 0, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0);
                     if (d + 1 < P.max_depth) shade_back_kernel(guided, tex, sb)<<<sgrid, sb, 0, st>>>(P, q, d, s0);
                 })) return rc;
-            if (overlap) {
+            // (the last bounce has nothing to run beside)
+            if (overlap && d + 1 < P.max_depth) {
                 PT_CU(cudaEventRecord(wf.fork, st));
                 PT_CU(cudaStreamWaitEvent(wf.side, wf.fork, 0));
                 shadow(wf.side);
@@ -1547,7 +1548,6 @@ int enqueue_batch(Wavefront& wf, const WaveParams& P, int64_t total_samples, cud
                 return rc;
             }
         }
-        if (overlap && P.max_depth > 0) PT_CU(cudaStreamWaitEvent(st, wf.join, 0));
         if (int rc = timed(3, [&] { k_finalize<<<wf.grid_finalize, 256, 0, st>>>(P, s0, count); })) return rc;
         if (train) {
             if (int rc = timed(4, [&] {
