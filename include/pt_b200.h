@@ -331,7 +331,9 @@ int         pt_integrator_destroy(pt_integrator* integ);
 const char* pt_integrator_name(const pt_integrator* integ);                       /* "Path" */
 /* Integrator::launch: trace params->sample_per_frame samples per pixel with the
  * scene's current frame count and fold them into the film.  Asynchronous on
- * `stream` (a cudaStream_t; NULL = the integrator's own stream). */
+ * `stream` (a cudaStream_t; NULL = the integrator's own stream).  Without
+ * PT_FLAG_NO_GRAPH the legacy default stream, and a stream that is being
+ * captured, are refused: a launch that comes again becomes a CUDA graph. */
 int pt_integrator_launch(pt_integrator* integ, pt_film* film, pt_scene* scene,
                          const pt_scene_params* params, void* stream);
 int pt_integrator_stats(const pt_integrator* integ, pt_render_stats* out);
@@ -339,7 +341,7 @@ int pt_integrator_reset_stats(pt_integrator* integ);
 
 /* ---- renderer (Renderer, Part_2/src/renderer.h:17-55) ---- */
 int pt_renderer_render_batch(pt_integrator* integ, pt_film* film, pt_scene* scene, void* stream); /* renderBatch */
-/* Added: `frames` consecutive renderBatch calls in one launch (one CUDA graph);
+/* Added: `frames` consecutive renderBatch calls in one launch;
  * identical film, frame counter and "new" image (the last frame's). */
 int pt_renderer_render_frames(pt_integrator* integ, pt_film* film, pt_scene* scene, uint32_t frames,
                               void* stream);
