@@ -111,7 +111,7 @@ int main(int argc, char** argv) {
 def walk(tmp_path_factory):
     d = tmp_path_factory.mktemp("wide_rays")
     (d / "rays.cpp").write_text(PROGRAM)
-    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-mfma", str(d / "rays.cpp"),
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", str(d / "rays.cpp"),
                     "-I", os.path.join(ROOT, "pathtracingtutorial_b200", "csrc"),
                     "-I", "/usr/local/cuda/include", "-o", str(d / "rays")], check=True)
 
